@@ -2849,9 +2849,12 @@ int bine_link_bytes(bine_comm_t comm, bine_coll_t coll, long count, bine_datatyp
     const Torus& t = comm->planner->torus();
     const size_t nlinks = (size_t)t.size * t.ndims * 2;
     unsigned long long* links = (unsigned long long*)d_link_bytes;
-    CUDA_TRY(cudaMemsetAsync(links, 0, nlinks * sizeof(unsigned long long), comm->stream));
     bool all_p2 = true;
-    for (int d = 0; d < t.ndims; d++) all_p2 &= is_pow2(t.dims[d]);
+    int max_ring = 1;
+    for (int d = 0; d < t.ndims; d++) {
+        all_p2 &= is_pow2(t.dims[d]);
+        max_ring = std::max(max_ring, t.dims[d]);
+    }
     const CollCfg& cf = comm->cfg[coll];
     bool mirrored = false;
     for (int p = 0; p < comm->ports; p++) mirrored |= mirrored_port(p, t.ndims);
@@ -2866,8 +2869,21 @@ int bine_link_bytes(bine_comm_t comm, bine_coll_t coll, long count, bine_datatyp
         else if (cl == kAllgather && cf.variant == kAgContPermute && cf.distance == kDecreasing)
             kind = 2;
     }
+    const dev::LinkGen g{t, cf.family, comm->ports, kind, (long long)count, es};
+    if (kind >= 0 && max_ring <= dev::kLinkMaxRing) {
+        // One block per ring, writing every link of the ring.
+        long long rings = 0;
+        for (int d = 0; d < t.ndims; d++) rings += t.size / t.dims[d];
+        const size_t smem = (size_t)max_ring * 24;
+        if (smem > 40 * 1024)
+            CUDA_TRY(cudaFuncSetAttribute(dev::k_link_rings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const int threads = std::min(1024, (max_ring + 31) / 32 * 32);
+        dev::k_link_rings<<<(unsigned)rings, threads, smem, comm->stream>>>(g, max_ring, links);
+        CUDA_TRY(cudaGetLastError());
+        return BINE_SUCCESS;
+    }
+    CUDA_TRY(cudaMemsetAsync(links, 0, nlinks * sizeof(unsigned long long), comm->stream));
     if (kind >= 0) {
-        dev::LinkGen g{t, cf.family, comm->ports, kind, (long long)count, es};
         const long long threads = (long long)t.size * comm->ports;
         unsigned grid = (unsigned)std::max(1LL, std::min((threads + 127) / 128, (long long)comm->num_sms * 32));
         dev::k_link_generate<<<grid, 128, 0, comm->stream>>>(g, links);

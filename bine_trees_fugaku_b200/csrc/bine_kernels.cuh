@@ -1691,6 +1691,235 @@ __global__ void k_link_generate(LinkGen g, unsigned long long* diff) {
     }
 }
 
+// The same schedules ring by ring, for tori whose rings hold at most
+// kLinkMaxRing nodes: one block per ring (a torus line of dimension d), in
+// one launch that writes every link once.
+//
+// Every message of these schedules moves along one dimension, so a ring's
+// link loads depend only on the messages between its own nodes.  At step k
+// of dimension d node p exchanges with q = peer_k(p) and q with p (the step
+// is an involution), so the difference entries at p come from p's own
+// message and the one it receives: each thread adds both to its own
+// entries, with no atomics, and a block scan turns them into loads.
+//
+// Message sizes of kind 0 need, per node, the number of ranks below `rem`
+// (the blocks one element longer) in the subtree it reaches with the steps
+// after k.  That subtree is a product over the dimensions of one-dimensional
+// subtrees (a step of one dimension leaves the other coordinates alone), and
+// "below rem" is lexicographic in the coordinates, so
+//
+//   f = sum over dims e of prod_{e' < e} M_e' * G_e * prod_{e' > e} Z_e'
+//
+// with G_e the members of dimension e's subtree below rem's coordinate, M_e
+// those equal to it and Z_e its size.  G and M obey G_k(c) = G_{k+1}(c) +
+// G_{k+1}(peer_k(c)), one addition per node and step, in place in shared
+// memory.
+//
+// k_link_generate walks each subtree node by node instead (P nodes per rank,
+// a serial chain on a local stack) and adds with global atomics, after a
+// memset and before k_link_scan.  It took 4,788 us of device time on the
+// 64x64 torus (allreduce B, 1 port) and the scan 48 us, 4,827 us per call;
+// with this kernel a call takes 16.4 us, bound by the latency of its steps
+// (a barrier pair and some hundred instructions each, 18 of them there).
+// The walk remains for rings beyond kLinkMaxRing, whose tables do not fit
+// in shared memory (24 bytes per node).
+constexpr int kLinkMaxRing = 8192;
+
+// Peer of coordinate c at a step of signed distance `dist` (Bine; negated
+// for odd coordinates) or of XOR distance `dist` (recursive doubling).
+__device__ __forceinline__ int ring_peer(bool xored, int dist, int L, int c) {
+    return xored ? c ^ dist : (c + ((c & 1) ? -dist : dist)) & (L - 1);
+}
+
+__global__ void __launch_bounds__(1024) k_link_rings(LinkGen g, int maxring, unsigned long long* __restrict__ links) {
+    extern __shared__ unsigned long long ring_smem[];
+    unsigned long long* dplus = ring_smem;        // + direction: difference entry of position p
+    unsigned long long* dminus = dplus + maxring;  // - direction: difference entry of position p + 1
+    int* cnt = (int*)(dminus + maxring);           // G of the current dimension at the current step
+    int* mem = cnt + maxring;                      // M
+    __shared__ StepDim sd[kMaxSteps];
+    __shared__ int8_t after[kMaxSteps][kMaxDims];  // steps of each dimension among steps 0..i
+    __shared__ int8_t at[kMaxDims][kMaxSteps];     // global step of (dimension, step)
+    __shared__ int dist[kMaxSteps];                // of a ring's step k on the current port
+    __shared__ int tabg[kMaxDims][kMaxSteps + 1], tabm[kMaxDims][kMaxSteps + 1];
+    __shared__ unsigned long long wsum[4][32];
+    const Torus& t = g.t;
+    const int S = t.num_steps, tid = threadIdx.x, nth = blockDim.x;
+    // The ring: dimension d, the other coordinates in c.
+    int line = blockIdx.x, d = 0;
+    while (d + 1 < t.ndims && line >= t.size / t.dims[d]) line -= t.size / t.dims[d++];
+    int c[kMaxDims] = {0, 0, 0};
+    for (int i = t.ndims - 1; i >= 0; i--) {
+        if (i == d) continue;
+        c[i] = line % t.dims[i];
+        line /= t.dims[i];
+    }
+    const int L = t.dims[d], Lm = L - 1;  // every dimension is a power of two here
+    const bool xored = g.family == kFamilyRecDoub;
+    for (int p = tid; p < L; p += nth) dplus[p] = dminus[p] = 0;
+    unsigned long long wp = 0, wm = 0;  // bytes of this thread's ranges that pass position 0
+    for (int port = 0; port < g.ports; port++) {
+        const long long cp = g.count / g.ports + (port < g.count % g.ports ? 1 : 0);
+        const long long q0 = cp >> S;  // 2^S ranks
+        const int rem = (int)(cp & (t.size - 1));
+        const bool uneven = g.kind == 0 && rem > 0;
+        int R[kMaxDims] = {0, 0, 0};
+        t.coords(rem, R);
+        __syncthreads();  // the previous port's tables are consumed
+        if (tid >= 32 - kMaxSteps && tid < 32) {
+            const int k = tid - (32 - kMaxSteps);
+            dist[k] = xored ? 1 << k : (mirrored_port(port, t.ndims) ? -rho(k) : rho(k));
+        }
+        if (tid == 0) {
+            step_dims(t, port, sd);
+            int8_t n[kMaxDims] = {0, 0, 0};
+            for (int i = 0; i < S; i++) {
+                at[sd[i].d][sd[i].k] = (int8_t)i;
+                n[sd[i].d]++;
+                for (int e = 0; e < kMaxDims; e++) after[i][e] = n[e];
+            }
+        }
+        // One dimension's G and M after every step, last step first: the
+        // other dimensions' at this ring's coordinates go to the tables.
+        auto begin = [&](int e) {
+            for (int p = tid; p < t.dims[e]; p += nth) {
+                cnt[p] = p < R[e];
+                mem[p] = p == R[e];
+            }
+            __syncthreads();
+        };
+        auto advance = [&](int e, int k) {
+            for (int p = tid; p < t.dims[e]; p += nth) {
+                const int q = ring_peer(xored, dist[k], t.dims[e], p);
+                if (p < q) {
+                    cnt[p] = cnt[q] = cnt[p] + cnt[q];
+                    mem[p] = mem[q] = mem[p] + mem[q];
+                }
+            }
+            __syncthreads();
+        };
+        if (uneven) {
+            for (int e = 0; e < t.ndims; e++) {
+                if (e == d) continue;
+                begin(e);
+                for (int k = t.steps_per_dim[e]; k >= 0; k--) {
+                    if (tid == 0) {
+                        tabg[e][k] = cnt[c[e]];
+                        tabm[e][k] = mem[c[e]];
+                    }
+                    if (k > 0) {
+                        __syncthreads();
+                        advance(e, k - 1);
+                    }
+                }
+                __syncthreads();  // cnt and mem are reused for the next dimension
+            }
+            begin(d);
+        } else {
+            __syncthreads();
+        }
+        for (int k = t.steps_per_dim[d] - 1; k >= 0; k--) {
+            const int i = at[d][k];
+            // f(x) = alpha * G(x) + beta * M(x) + gamma at this step.
+            long long alpha = 0, beta = 0, gamma = 0;
+            if (uneven) {
+                long long pre = 1, pre_d = 1;  // products of M: all dims before e; without dimension d
+                for (int e = 0; e < t.ndims; e++) {
+                    long long post = 1;
+                    for (int h = e + 1; h < t.ndims; h++) post <<= t.steps_per_dim[h] - after[i][h];
+                    if (e == d) {
+                        alpha = pre * post;
+                    } else {
+                        const int ke = after[i][e];
+                        if (e < d) gamma += pre * tabg[e][ke] * post;
+                        else beta += pre_d * tabg[e][ke] * post;
+                        if (e < d) pre *= tabm[e][ke];
+                        pre_d *= tabm[e][ke];
+                    }
+                }
+            }
+            for (int p = tid; p < L; p += nth) {
+                const int q = ring_peer(xored, dist[k], L, p);
+                unsigned long long bytes;
+                if (g.kind == 1) {
+                    bytes = (unsigned long long)cp;
+                } else if (g.kind == 2) {
+                    bytes = (unsigned long long)cp << (S - 1 - i);
+                } else {  // the reduce-scatter message one way and the allgather's from the peer
+                    bytes = 2ull * ((unsigned long long)q0 << (S - 1 - i));
+                    if (uneven) bytes += alpha * (cnt[p] + cnt[q]) + beta * (mem[p] + mem[q]) + 2 * gamma;
+                }
+                bytes *= g.es;
+                // p's message to q takes the shorter way round (+ on ties),
+                // and so does q's to p.
+                const int h = (q - p) & Lm;
+                unsigned long long dp = 0, dm = 0;
+                if (h + h <= L) {  // + : positions p .. p + h - 1
+                    dp += bytes;
+                    if (p + h >= L) wp += bytes;
+                } else {  // - : positions q + 1 .. p
+                    dm -= bytes;
+                    if (((q + 1) & Lm) + (L - h) >= L) wm += bytes;
+                }
+                if (h + h >= L) dp -= bytes;  // q's message comes in the + direction and ends before p
+                else dm += bytes;             // or in the - direction, from position p + 1 on
+                dplus[p] += dp;
+                dminus[p] += dm;
+            }
+            if (uneven && k > 0) {
+                __syncthreads();
+                advance(d, k);
+            }
+        }
+    }
+    __syncthreads();
+    // Scan: thread tid owns positions [tid * per, +per).
+    const int per = (L + nth - 1) / nth, p0 = min(L, tid * per), p1 = min(L, p0 + per);
+    unsigned long long sp = 0, sm = 0;
+    for (int p = p0; p < p1; p++) {
+        sp += dplus[p];
+        sm += dminus[p];
+    }
+    const int lane = tid & 31, warp = tid >> 5;
+    unsigned long long ip = sp, im = sm;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long a = __shfl_up_sync(0xffffffffu, ip, o), b = __shfl_up_sync(0xffffffffu, im, o);
+        if (lane >= o) {
+            ip += a;
+            im += b;
+        }
+        wp += __shfl_xor_sync(0xffffffffu, wp, o);
+        wm += __shfl_xor_sync(0xffffffffu, wm, o);
+    }
+    if (lane == 31) {
+        wsum[0][warp] = ip;
+        wsum[1][warp] = im;
+        wsum[2][warp] = wp;
+        wsum[3][warp] = wm;
+    }
+    __syncthreads();
+    unsigned long long ap = ip - sp, am = im - sm;  // exclusive prefixes
+    unsigned long long tp = 0, tm = dminus[L - 1];
+    for (int w = 0; w < nth / 32; w++) {
+        if (w < warp) {
+            ap += wsum[0][w];
+            am += wsum[1][w];
+        }
+        tp += wsum[2][w];
+        tm += wsum[3][w];
+    }
+    size_t li = link_index(t, t.id(c), d, 0);  // c[d] = 0: position 0
+    size_t step = 2 * t.ndims;                 // links of consecutive positions
+    for (int e = d + 1; e < t.ndims; e++) step *= t.dims[e];
+    for (int p = p0; p < p1; p++) {
+        ap += dplus[p];
+        links[li + p * step] = tp + ap;      // prefix including position p
+        links[li + p * step + 1] = tm + am;  // entries of positions 0..p, each one place to the left
+        am += dminus[p];
+    }
+}
+
 // One thread per ring: prefix sums of the difference array, in place.
 __global__ void k_link_scan(Torus t, unsigned long long* links) {
     long long nlines = 0;
