@@ -894,6 +894,46 @@ bool flat_tables(const TreePlan& tp, const SplitTrees& st, const SplitTrees* se,
     return true;
 }
 
+// Lanes per output vector of the exact-order float kernels for one call:
+// more than one when the output has too few vectors to fill the GPU several
+// times over.  *leaves: the smallest tree.
+int tree_lanes(bine_comm_t c, const TreePlan& tp, int64_t L, int* leaves) {
+    int min_leaves = INT32_MAX;  // one leaf per entry
+    int64_t vecs = 0;
+    for (const OutSegment& sg : tp.segs) {
+        if (sg.n <= 0) continue;
+        min_leaves = std::min(min_leaves, sg.prog_len);
+        vecs += sg.n / L;
+    }
+    int K = 1;
+    if (c->tree_split > 0) {
+        K = c->tree_split;
+        while (K > 1 && min_leaves < K) K /= 2;
+    } else {
+        // By P, as measured on B200 at 2-4 MiB per rank (GB/s for 1 / 2
+        // / 4 / 8 warps per vector group): P = 64: 4649 / 5424 / 5001 /
+        // 4407; P = 96: 3508 / 4566 / 4165 / 3661; P = 256: 5481 / 5843 /
+        // 6026 / 5879; P = 384: 4023 / 4244 / 4216 / 4065; P = 1000:
+        // 2805 / 2825 / 2898 / 3372.
+        const int P = c->P;
+        K = P < 32 ? 1 : (P < 128 ? 2 : (P < 512 ? 4 : 8));
+        // Calls with few output vectors: more lanes per vector until
+        // vectors x lanes reach a parallelism target that grows with
+        // the tree (2^17 lanes up to P = 128, proportionally above),
+        // keeping at least 4 leaves per lane.  Measured on B200
+        // (float32, us per call, automatic rule before -> after):
+        // P = 96 at 128 KiB / 512 KiB per rank: 21.3 -> 12.1 / 39.0 ->
+        // 24.6; P = 384: 51.2 -> 41.0 / 128.2 -> 100.1; P = 64 at
+        // 128 KiB: 12.3 -> 8.2.  From 2 MiB per rank the rule by P
+        // stands.
+        const int64_t target = (int64_t)1 << 17 < (int64_t)1024 * P ? (int64_t)1024 * P : (int64_t)1 << 17;
+        while (K < 8 && 8 * K <= P && vecs * K < target) K *= 2;
+    }
+    while (K > 1 && min_leaves < 2 * K) K /= 2;  // 2K parts of at least one leaf
+    *leaves = min_leaves;
+    return K;
+}
+
 // With `dry` the call plans the trees and their tile lists on the host and
 // uploads nothing (no device is needed; the result is not cached and its
 // device pointers stay null): bine_plan_tree_form reports from it.
@@ -941,16 +981,11 @@ int get_dev_trees(bine_comm_t c, const PlanKey& k, int es, std::shared_ptr<DevTr
     }
     // Every segment whose program reads at 16-byte-aligned shifts gets a
     // vector body: its elements from the first to the last 16-byte boundary
-    // of the output row.  Heads, tails and the other segments run through
-    // the element kernel (rtiles); atiles cover everything element-wise for
-    // layouts that are not 16-byte aligned.
+    // of the output row.  Heads, tails and the other segments run as element
+    // tiles (rtiles); atiles cover everything so for layouts that are not
+    // 16-byte aligned.
     const int64_t L = 16 / es;
     std::vector<int64_t> body_lo(tp.segs.size(), 0), body_hi(tp.segs.size(), 0);
-    std::vector<dev::TreeTile> tiles, rtiles, htiles, atiles;
-    const int64_t vtile = (int64_t)dev::kThreads * L, etile = (int64_t)dev::kThreads * 4;
-    auto add_tiles = [](std::vector<dev::TreeTile>* v, int32_t seg, int64_t lo, int64_t hi, int64_t step) {
-        for (int64_t st = lo; st < hi; st += step) v->push_back(dev::TreeTile{seg, 0, st, std::min(step, hi - st)});
-    };
     for (size_t i = 0; i < tp.segs.size(); i++) {
         const OutSegment& sg = tp.segs[i];
         bool pv = true;
@@ -962,6 +997,17 @@ int get_dev_trees(bine_comm_t c, const PlanKey& k, int es, std::shared_ptr<DevTr
                 body_hi[i] = hi;
             }
         }
+    }
+    int min_leaves = 0;
+    const int K = tree_lanes(c, tp, L, &min_leaves);
+    std::vector<dev::TreeTile> tiles, rtiles, htiles, atiles;
+    // Element tiles are as wide as K lanes per vector leave (k_tree_strided).
+    const int64_t vtile = (int64_t)dev::kThreads * L, etile = vtile / K;
+    auto add_tiles = [](std::vector<dev::TreeTile>* v, int32_t seg, int64_t lo, int64_t hi, int64_t step) {
+        for (int64_t st = lo; st < hi; st += step) v->push_back(dev::TreeTile{seg, 0, st, std::min(step, hi - st)});
+    };
+    for (size_t i = 0; i < tp.segs.size(); i++) {
+        const OutSegment& sg = tp.segs[i];
         add_tiles(&tiles, (int32_t)i, body_lo[i], body_hi[i], vtile);
         // Element pieces shorter than one vector go to the staged kernel.
         auto piece = [&](int64_t lo, int64_t hi) { add_tiles(hi - lo < L ? &htiles : &rtiles, (int32_t)i, lo, hi, etile); };
@@ -1015,40 +1061,9 @@ int get_dev_trees(bine_comm_t c, const PlanKey& k, int es, std::shared_ptr<DevTr
     if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess || e5 != cudaSuccess ||
         e6 != cudaSuccess)
         return fail(BINE_ERR_CUDA, "uploading the reduction trees failed");
-    // Split form of the vector bodies: K lanes per output vector when the
-    // output has too few vectors to fill the GPU several times over.
-    if (!tiles.empty()) {
-        int min_leaves = INT32_MAX;
-        for (size_t i = 0; i < tp.segs.size(); i++)
-            if (body_lo[i] < body_hi[i]) min_leaves = std::min(min_leaves, tp.segs[i].prog_len);  // one leaf per entry
-        int K = 1;
-        if (c->tree_split > 0) {
-            K = c->tree_split;
-            while (K > 1 && min_leaves < K) K /= 2;
-        } else {
-            // By P, as measured on B200 at 2-4 MiB per rank (GB/s for 1 / 2
-            // / 4 / 8 warps per vector group): P = 64: 4649 / 5424 / 5001 /
-            // 4407; P = 96: 3508 / 4566 / 4165 / 3661; P = 256: 5481 / 5843 /
-            // 6026 / 5879; P = 384: 4023 / 4244 / 4216 / 4065; P = 1000:
-            // 2805 / 2825 / 2898 / 3372.
-            const int P = c->P;
-            K = P < 32 ? 1 : (P < 128 ? 2 : (P < 512 ? 4 : 8));
-            // Calls with few output vectors: more lanes per vector until
-            // vectors x lanes reach a parallelism target that grows with
-            // the tree (2^17 lanes up to P = 128, proportionally above),
-            // keeping at least 4 leaves per lane.  Measured on B200
-            // (float32, us per call, automatic rule before -> after):
-            // P = 96 at 128 KiB / 512 KiB per rank: 21.3 -> 12.1 / 39.0 ->
-            // 24.6; P = 384: 51.2 -> 41.0 / 128.2 -> 100.1; P = 64 at
-            // 128 KiB: 12.3 -> 8.2.  From 2 MiB per rank the rule by P
-            // stands.
-            int64_t vecs = 0;
-            for (size_t i = 0; i < tp.segs.size(); i++) vecs += (body_hi[i] - body_lo[i]) / L;
-            const int64_t target = (int64_t)1 << 17 < (int64_t)1024 * P ? (int64_t)1024 * P : (int64_t)1 << 17;
-            while (K < 8 && 8 * K <= P && vecs * K < target) K *= 2;
-        }
-        while (K > 1 && min_leaves < 2 * K) K /= 2;  // 2K parts of at least one leaf
-        if (K > 1) {
+    // Split form: K lanes per output vector.
+    if (K > 1) {
+        {
             // K parts, one per warp, or 2K parts assigned longest first when
             // that lowers the busiest warp's leaves by 5 % or more (trees of
             // non-power-of-two P do not cut into K equal subtrees).
@@ -1337,6 +1352,28 @@ int launch_tree_split(bine_comm_t c, const DevTrees& d, const char* in, long lon
     return BINE_SUCCESS;
 }
 
+// Element tiles (at most kThreads / K lane vectors each) of layouts and
+// segments off the 16-byte grid.
+template <typename T, int K>
+int launch_tree_strided(bine_comm_t c, const DevTrees& d, const char* in, long long ist, char* out, long long ost,
+                        const dev::TreeTile* tiles, int ntiles, cudaStream_t s) {
+    const bool split = K > 1;
+    const TreeSmem sm = tree_smem(split ? d.smax_prog_len : d.max_prog_len, split ? d.sdepth : d.depth);
+    auto kern = sm.stack ? dev::k_tree_strided<T, K, true> : dev::k_tree_strided<T, K, false>;
+    unsigned g = 0;
+    int rc = launch_tree_kernel(c, kern, sm.bytes, ntiles, &g);
+    if constexpr (K > 1) {
+        // The largest programs leave no room for the parts' partial sums.
+        if (rc == BINE_ERR_UNSUPPORTED) return launch_tree_strided<T, 1>(c, d, in, ist, out, ost, tiles, ntiles, s);
+    }
+    if (rc) return rc;
+    kern<<<g, dev::kThreads, sm.bytes, s>>>(in, ist, out, ost, c->P, split ? d.ssegs : d.segs,
+                                            split ? d.sprog : d.prog, d.sparts, d.scomb, d.sassign, tiles, ntiles,
+                                            split ? d.split_parts : 1, sm.stack_off);
+    CUDA_TRY(cudaGetLastError());
+    return BINE_SUCCESS;
+}
+
 // Arguments and dynamic shared memory of the row-aligned kernels: the
 // common additions, the ranks of up to `fmax_ns` segments (row tiles only),
 // then the evaluation stacks when they fit.
@@ -1442,8 +1479,8 @@ TileSet all_tiles(const DevTrees& d) {
 // column window's).  On a 16-byte-aligned layout the vector tiles (split
 // form when the plan has one) run on the communicator's stream while the
 // element pieces run beside them on a side stream (forked and joined by
-// events, which graph capture also records); otherwise every element tile
-// runs on the element kernel.
+// events, which graph capture also records); otherwise every segment runs as
+// strided element tiles.
 template <typename T>
 int launch_tree(bine_comm_t c, const DevTrees& d, const char* in, long long ist, char* out, long long ost,
                 const TileSet& ts) {
@@ -1451,12 +1488,16 @@ int launch_tree(bine_comm_t c, const DevTrees& d, const char* in, long long ist,
     unsigned g = 0;
     int rc;
     const bool edges = vec && d.flat && ts.n[5] > 0;
-    const bool side = vec && (ts.n[2] > 0 || ts.n[3] > 0 || edges);
+    const bool pieces = vec && (ts.n[2] > 0 || ts.n[3] > 0 || edges);
+    // Beside vector tiles only: pieces alone need no second stream.
+    const bool side = pieces && (d.split_k > 1 ? ts.n[1] : ts.n[0]) > 0;
     cudaStream_t es = c->stream;
     if (side) {
         CUDA_TRY(cudaEventRecord(c->ev_fork, c->stream));
         CUDA_TRY(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
         es = c->side;
+    }
+    if (pieces) {
         if (edges) {
             rc = launch_tree_edges<T>(c, d, in, ist, out, ost, ts.edge0, ts.n[5], es);
             if (rc) return rc;
@@ -1504,11 +1545,13 @@ int launch_tree(bine_comm_t c, const DevTrees& d, const char* in, long long ist,
     const dev::TreeTile* et = vec ? ts.t[2] : ts.t[4];
     const int ne = vec ? ts.n[2] : ts.n[4];
     if (ne > 0) {
-        const size_t smem = (size_t)std::max(1, d.max_prog_len) * sizeof(dev::TreeEntry);
-        rc = launch_tree_kernel(c, dev::k_tree_scalar<T>, smem, ne, &g);
+        switch (d.split_k) {
+        case 1: rc = launch_tree_strided<T, 1>(c, d, in, ist, out, ost, et, ne, es); break;
+        case 2: rc = launch_tree_strided<T, 2>(c, d, in, ist, out, ost, et, ne, es); break;
+        case 4: rc = launch_tree_strided<T, 4>(c, d, in, ist, out, ost, et, ne, es); break;
+        default: rc = launch_tree_strided<T, 8>(c, d, in, ist, out, ost, et, ne, es); break;
+        }
         if (rc) return rc;
-        dev::k_tree_scalar<T><<<g, dev::kThreads, smem, es>>>(in, ist, out, ost, c->P, d.segs, d.prog, et, ne);
-        CUDA_TRY(cudaGetLastError());
     }
     if (side) {
         CUDA_TRY(cudaEventRecord(c->ev_join, c->side));
@@ -2619,7 +2662,7 @@ int bine_plan_tree_form(bine_comm_t comm, bine_coll_t coll, long count, bine_dat
     int rc = get_dev_trees(comm, make_key(comm, coll, count, root), dtype_size(datatype), &d, true);
     if (rc) return rc;
     out[0] = d->flat ? 3 : (d->split_k > 1 && d->nstiles > 0 ? 2 : (d->ntiles > 0 ? 1 : 0));
-    out[1] = d->split_k;
+    out[1] = d->nstiles > 0 ? d->split_k : 1;  // lanes of the vector tiles
     out[2] = d->flat ? d->fnshape : 0;
     out[3] = d->split_k > 1 ? d->nstiles : d->ntiles;
     out[4] = d->flat ? d->nfedges : 0;

@@ -58,6 +58,48 @@ __device__ __forceinline__ void st_stream(void* p, uint4 v) {
                  : "memory");
 }
 
+// Strided lane vectors, for rows that do not share a 16-byte grid (packed
+// rows of odd length, blocks of odd length): the 16 / sizeof(T) elements of
+// a lane lie `STEP` elements apart and consecutive lanes hold consecutive
+// elements, so every access of a warp is a run of 32 elements wherever the
+// row starts, and the vector arithmetic stays that of the 16-byte form.
+// `n` elements of the vector exist (the first ones); the others read as 0.
+template <typename T>
+__device__ __forceinline__ T ld_stream_elem(const void* p) {
+    T v;
+    if constexpr (sizeof(T) == 8) {
+        unsigned long long r;
+        asm volatile("ld.global.nc.L1::no_allocate.u64 %0, [%1];" : "=l"(r) : "l"(p));
+        memcpy(&v, &r, 8);
+    } else if constexpr (sizeof(T) == 4) {
+        unsigned r;
+        asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(r) : "l"(p));
+        memcpy(&v, &r, 4);
+    } else {
+        unsigned r;
+        asm volatile("ld.global.nc.L1::no_allocate.u8 %0, [%1];" : "=r"(r) : "l"(p));
+        v = (T)r;
+    }
+    return v;
+}
+template <typename T, int STEP>
+__device__ __forceinline__ uint4 ld_strided(const char* p, int n) {
+    constexpr int N = 16 / sizeof(T);
+    uint4 raw;
+    T* t = reinterpret_cast<T*>(&raw);
+#pragma unroll
+    for (int i = 0; i < N; i++) t[i] = i < n ? ld_stream_elem<T>(p + i * STEP * (int)sizeof(T)) : (T)0;
+    return raw;
+}
+template <typename T, int STEP>
+__device__ __forceinline__ void st_strided(char* p, uint4 raw, int n) {
+    constexpr int N = 16 / sizeof(T);
+    const T* t = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        if (i < n) __stcs(reinterpret_cast<T*>(p) + i * STEP, t[i]);
+}
+
 // ----------------------------------------------------------- lane algebra
 // Accumulators: wrapping integers of the element type, FP64 for the FAST
 // float order, the element type itself for the exact float order.
@@ -335,11 +377,11 @@ struct TreeComb {  // combine entry: push part `part`, then `adds` additions
     int32_t part, adds;
 };
 
-// Evaluates program entries [b, b + len) for one 16-byte vector whose first
-// input element is at `base` (entries hold each leaf's byte offset from
-// there), loads kRing entries ahead of the additions.
-template <typename T, bool SMEM, int kRing>
-__device__ __forceinline__ uint4 eval_program(const char* __restrict__ base, const TreeEntry* sprog, int b, int len,
+// Evaluates program entries [b, b + len) for one lane vector; `ld` loads it
+// at a leaf's byte offset (entries hold it precomputed), kRing entries ahead
+// of the additions.
+template <typename T, bool SMEM, int kRing, typename Ld>
+__device__ __forceinline__ uint4 eval_program(const Ld& ld, const TreeEntry* sprog, int b, int len,
                                               EvalStack<SMEM>& stk) {
     uint4 top = make_uint4(0, 0, 0, 0);
     int sp = 0;
@@ -348,7 +390,7 @@ __device__ __forceinline__ uint4 eval_program(const char* __restrict__ base, con
     for (int u = 0; u < kRing; u++)
         if (u < len) {
             const TreeEntry q = sprog[b + u];
-            ring[u] = ld_stream(base + q.shift);
+            ring[u] = ld(q.shift);
         }
     for (int k0 = 0; k0 < len; k0 += kRing) {
 #pragma unroll
@@ -358,7 +400,7 @@ __device__ __forceinline__ uint4 eval_program(const char* __restrict__ base, con
                 const uint4 v = ring[u];
                 if (k + kRing < len) {
                     const TreeEntry q = sprog[b + k + kRing];
-                    ring[u] = ld_stream(base + q.shift);
+                    ring[u] = ld(q.shift);
                 }
                 if (k > 0) stk.set(sp++, top);
                 top = v;
@@ -419,8 +461,9 @@ __global__ void __launch_bounds__(kThreads) k_tree_split(const char* __restrict_
         if (active) {
             for (int pi = sasg[nparts + j]; pi < sasg[nparts + j + 1]; pi++) {
                 const int p = sasg[pi];
-                partial[g][p][lane] = eval_program<T, SMEM, 4>(in + e * (long long)sizeof(T), sprog, spart[p],
-                                                               spart[p + 1] - spart[p], stk);
+                const char* base = in + e * (long long)sizeof(T);
+                partial[g][p][lane] = eval_program<T, SMEM, 4>([&](long long off) { return ld_stream(base + off); },
+                                                               sprog, spart[p], spart[p + 1] - spart[p], stk);
             }
         }
         __syncthreads();
@@ -792,37 +835,94 @@ __global__ void __launch_bounds__(kThreads) k_tree_staged(const char* __restrict
     }
 }
 
-// Element form for layouts that are not 16-byte aligned.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_tree_scalar(const char* __restrict__ in, long long in_stride,
-                                                          char* __restrict__ out, long long out_stride, int P,
-                                                          const TreeSeg* __restrict__ segs,
-                                                          const TreeEntry* __restrict__ prog,
-                                                          const TreeTile* __restrict__ tiles, int ntiles) {
-    extern __shared__ TreeEntry sprog[];
+// Form for layouts and segments off the 16-byte grid (packed rows of odd
+// length, blocks of odd length): k_tree_split over strided lane vectors.  A
+// tile is up to (8 / K) groups of 32 lanes times 16 / sizeof(T) elements of
+// one segment; element i of a lane's vector lies 32 * i elements after its
+// first, so every load and store of a warp is one run of 32 elements.  K = 1
+// evaluates whole programs (no split plan).
+//
+// Bound by HBM like the aligned form (the arithmetic per row is the same,
+// with four 4-byte loads in the place of one of 16).  It replaced a kernel
+// of one element per thread and one load in flight on 1,024-element tiles
+// (288 blocks): float32 allreduce at P = 96, 262,147 elements per rank,
+// 232 -> 44.3 us per call (867 -> 4,550 GB/s); P = 256 at 1,048,579
+// elements runs at 5,180 GB/s, reduce_scatter at P = 64 and 32,769 at 5,530.
+template <typename T, int K, bool SMEM>
+__global__ void __launch_bounds__(kThreads) k_tree_strided(const char* __restrict__ in, long long in_stride,
+                                                           char* __restrict__ out, long long out_stride, int P,
+                                                           const TreeSeg* __restrict__ segs,
+                                                           const TreeEntry* __restrict__ prog,
+                                                           const int* __restrict__ parts,
+                                                           const TreeComb* __restrict__ comb,
+                                                           const int* __restrict__ assign,
+                                                           const TreeTile* __restrict__ tiles, int ntiles,
+                                                           int nparts, int stack_off) {
+    extern __shared__ uint4 sdyn[];
+    TreeEntry* sprog = reinterpret_cast<TreeEntry*>(sdyn);
+    EvalStack<SMEM> stk;
+    stk.init(sdyn + stack_off);
+    constexpr int kWarps = kThreads / 32;
+    constexpr int kGroups = kWarps / K;
+    constexpr int KP = 2 * K;
+    __shared__ int spart[KP + 1];
+    __shared__ TreeComb scomb[KP];
+    __shared__ int sasg[KP + K + 1];
+    __shared__ uint4 partial[K > 1 ? kGroups : 1][K > 1 ? KP : 1][32];
+    constexpr int L = 16 / sizeof(T);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = warp % K, g = warp / K;
+    int cur = -1;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const TreeTile tile = tiles[t];
         const TreeSeg sg = segs[tile.seg];
-        __syncthreads();
-        for (int i = threadIdx.x; i < sg.prog_len; i += blockDim.x) sprog[i] = prog[sg.prog_begin + i];
-        __syncthreads();
-        for (long long col = threadIdx.x; col < tile.n; col += blockDim.x) {
-            const long long e = sg.off + tile.start + col;
-            T stk[kMaxTreeDepth];
-            T top = (T)0;
-            int sp = 0;
-            for (int k = 0; k < sg.prog_len; k++) {
-                const TreeEntry q = sprog[k];
-                const T v = *(const T*)(in + (long long)q.rank * in_stride + (e + q.shift) * (long long)sizeof(T));
-                if (k > 0) stk[sp++] = top;
-                top = v;
-                for (int a = q.adds; a > 0; a--) top = add_exact<T>(stk[--sp], top);
+        __syncthreads();  // the previous tile's partials and program are consumed
+        if (tile.seg != cur) {  // block-uniform
+            for (int i = threadIdx.x; i < sg.prog_len; i += blockDim.x) {
+                TreeEntry q = prog[sg.prog_begin + i];
+                q.shift = (long long)q.rank * in_stride + q.shift * (long long)sizeof(T);  // byte offset
+                sprog[i] = q;
             }
-            if (sg.rank < 0) {
-                for (int d = 0; d < P; d++) *(T*)(out + (long long)d * out_stride + e * (long long)sizeof(T)) = top;
-            } else {
-                *(T*)(out + (long long)sg.rank * out_stride + e * (long long)sizeof(T)) = top;
+            if constexpr (K > 1) {
+                if (threadIdx.x <= nparts) spart[threadIdx.x] = parts[(long long)tile.seg * (nparts + 1) + threadIdx.x];
+                if (threadIdx.x < nparts) scomb[threadIdx.x] = comb[(long long)tile.seg * nparts + threadIdx.x];
+                if (threadIdx.x < nparts + K + 1)
+                    sasg[threadIdx.x] = assign[(long long)tile.seg * (nparts + K + 1) + threadIdx.x];
             }
+            __syncthreads();
+            cur = tile.seg;
+        }
+        const long long col = (long long)g * (32 * L) + lane;  // first element of the lane's vector, in the tile
+        const int nact = (int)min((long long)L, (tile.n - col + 31) / 32);  // its elements inside the tile
+        const long long byte = (sg.off + tile.start + col) * (long long)sizeof(T);
+        const char* base = in + byte;
+        const auto ld = [&](long long off) { return ld_strided<T, 32>(base + off, nact); };
+        uint4 top = make_uint4(0, 0, 0, 0);
+        if constexpr (K > 1) {
+            if (nact > 0) {
+                for (int pi = sasg[nparts + j]; pi < sasg[nparts + j + 1]; pi++) {
+                    const int p = sasg[pi];
+                    partial[g][p][lane] = eval_program<T, SMEM, 4>(ld, sprog, spart[p], spart[p + 1] - spart[p], stk);
+                }
+            }
+            __syncthreads();
+            if (nact <= 0) continue;
+            int csp = 0;  // the parts' stack is empty again: the combine reuses it
+            for (int q = 0; q < nparts; q++) {
+                const TreeComb c = scomb[q];
+                if (q > 0) stk.set(csp++, top);
+                top = partial[g][c.part][lane];
+                for (int a = c.adds; a > 0; a--) top = vadd<T>(stk.get(--csp), top);
+            }
+        } else {
+            if (nact <= 0) continue;
+            top = eval_program<T, SMEM, 4>(ld, sprog, 0, sg.prog_len, stk);
+        }
+        char* o = out + byte;
+        if (sg.rank < 0) {
+            for (int d = j; d < P; d += K) st_strided<T, 32>(o + (long long)d * out_stride, top, nact);
+        } else if (j == 0) {
+            st_strided<T, 32>(o + (long long)sg.rank * out_stride, top, nact);
         }
     }
 }

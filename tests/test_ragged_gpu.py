@@ -1,0 +1,108 @@
+"""Rows and blocks off the 16-byte grid on the FUSED engine: packed rows of
+odd length, blocks of odd length, buffers that start in the middle of a
+vector.  Results are compared bit for bit with the oracle (floats in the
+reference's order) or with exact sums and copies, and the bytes around the
+receive rows stay as they were."""
+import numpy as np
+import pytest
+import torch
+
+import bine_trees_fugaku_b200 as bine
+from oracle import port
+from oracle.common import buffer_counts, expected
+
+pytestmark = pytest.mark.gpu
+
+CODE = {np.dtype(np.int32): bine.INT32, np.dtype(np.int64): bine.INT64, np.dtype(np.float32): bine.FLOAT,
+        np.dtype(np.float64): bine.DOUBLE, np.dtype(np.int8): bine.CHAR}
+GUARD = 64  # elements before and after the receive rows
+
+
+def values(shape, dtype, seed):
+    rng = np.random.default_rng(seed)
+    if np.dtype(dtype).kind == "f":
+        return rng.standard_normal(shape).astype(dtype)
+    lim = 100 if dtype == np.int8 else 1000
+    return rng.integers(-lim, lim + 1, shape).astype(dtype)
+
+
+def call(coll, x, count, shift=0, pad=0, variant=None, lanes=0, order="reference", root=0):
+    """The collective on rows `pad` elements longer than their data, in
+    buffers that start `shift` elements after a 16-byte boundary; checks the
+    guards and the padding."""
+    P = x.shape[0]
+    si, so = buffer_counts(coll, count, P)
+    td = torch.from_numpy(x[:1, :1]).dtype
+    comm = bine.Comm(P)
+    if variant:
+        comm.set_algo(coll, variant)
+    comm.set_tree_split(lanes)
+    comm.set_float_order(order)
+    comm.set_stream(torch.cuda.current_stream())
+    es = x.dtype.itemsize
+    send = torch.zeros(P * (si + pad) + shift + 1, dtype=td, device="cuda")
+    rows = send[shift:shift + P * (si + pad)].view(P, si + pad)
+    rows[:, :si] = torch.from_numpy(x).cuda()
+    recv = torch.full((P * (so + pad) + 2 * GUARD + shift,), 77, dtype=td, device="cuda")
+    out = recv[GUARD + shift:GUARD + shift + P * (so + pad)].view(P, so + pad)
+    if coll == "bcast":
+        out[root, :so] = rows[root, :si]
+    if pad:
+        comm.set_layout((si + pad) * es, (so + pad) * es)
+    comm.run(coll, rows, out, count, CODE[x.dtype], root)
+    comm.synchronize()
+    got = out[:, :so].cpu().numpy()
+    assert (out[:, so:] == 77).all()
+    assert (recv[:GUARD + shift] == 77).all() and (recv[GUARD + shift + P * (so + pad):] == 77).all()
+    comm.close()
+    return got
+
+
+def same_bits(a, b):
+    return np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("P,count,shift,pad", [
+    (4, 4, 1, 0), (6, 127, 0, 0), (16, 129, 0, 0), (16, 16 * 128 + 3, 1, 0), (24, 24 * 33 + 1, 0, 0),
+    (48, 48 * 129 - 1, 1, 0), (96, 96 * 257 + 5, 0, 0), (130, 130 * 40 + 7, 0, 3), (64, 64 * 512, 1, 1), (256, 256 * 21 + 1, 0, 0),
+    (520, 520 * 5 + 3, 0, 0)])
+def test_exact_order_allreduce_matches_the_oracle(P, count, shift, pad, dtype):
+    x = values((P, count), dtype, P + count)
+    want, _ = port.run("allreduce", x, count, variant="B")
+    assert same_bits(call("allreduce", x, count, shift, pad), want)
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("P,count", [(64, 64 * 130 + 1), (96, 96 * 600 + 3)])
+def test_every_lane_count_gives_the_same_bits(P, count, lanes):
+    x = values((P, count), np.float32, lanes)
+    want, _ = port.run("allreduce", x, count, variant="B")
+    assert same_bits(call("allreduce", x, count, lanes=lanes), want)
+
+
+def test_per_rank_trees_off_the_grid():
+    """The L butterfly's trees differ from rank to rank: one destination row
+    per segment."""
+    x = values((16, 259), np.float32, 3)
+    want, _ = port.run("allreduce", x, 259, variant="L")
+    assert same_bits(call("allreduce", x, 259, variant="L"), want)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("P,count,shift", [(4, 1, 0), (8, 3, 1), (16, 33, 0), (64, 129, 0), (64, 1025, 1), (128, 17, 0)])
+def test_exact_order_reduce_scatter_matches_the_oracle(P, count, shift, dtype):
+    if dtype == np.float64:  # the reference reduces no 64-bit types here: whole numbers, exact in any order
+        x = values((P, P * count), np.int32, P + count).astype(dtype)
+        want = expected("reduce_scatter", x, P, count)
+    else:
+        x = values((P, P * count), dtype, P + count)
+        want, _ = port.run("reduce_scatter", x, count)
+    assert same_bits(call("reduce_scatter", x, count, shift), want)
+
+
+@pytest.mark.parametrize("P,count,root", [(16, 1001, 0), (64, 64 * 65 + 3, 0)])
+def test_exact_order_reduce_matches_the_oracle(P, count, root):
+    x = values((P, count), np.float32, P)
+    want, _ = port.run("reduce", x, count, root=root)
+    assert same_bits(call("reduce", x, count, root=root)[root], want[root])
