@@ -1218,77 +1218,86 @@ unsigned resident_blocks(bine_comm_t c, K kern, int threads, size_t smem) {
     return (unsigned)(per_sm * std::max(1, c->num_sms));
 }
 
-template <typename T, int COLS>
+template <typename T, int COLS, bool VEC>
 int launch_sum_cols(bine_comm_t c, int mode, const char* in, long long ist, char* out, long long ost, int P,
-                    long long ncol, long long blk_vec, int root) {
+                    long long n, long long blk, int root, long long e0) {
     // One tile per block, up to 64 blocks per SM (then grid-stride): the
     // hardware scheduler back-fills SMs as blocks finish, where a single
     // resident wave walking the tiles leaves a tail (measured on B200, P =
     // 256, 4 MiB per rank: 5716 GB/s resident wave, 6347 one tile per
     // block).
-    const long long tiles = (ncol + COLS - 1) / COLS;
+    constexpr long long width = COLS * (16 / sizeof(T));
+    const long long tiles = (n + width - 1) / width;
     const unsigned g = (unsigned)std::min<long long>(tiles, 64LL * std::max(1, c->num_sms));
     if (mode == dev::kSumAllreduce)
-        dev::k_sum_vec<T, dev::kSumAllreduce, COLS><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, ncol,
-                                                                                         blk_vec, root);
+        dev::k_sum_vec<T, dev::kSumAllreduce, COLS, VEC><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, n,
+                                                                                              blk, root, e0);
     else if (mode == dev::kSumReduceScatter)
-        dev::k_sum_vec<T, dev::kSumReduceScatter, COLS><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P,
-                                                                                             ncol, blk_vec, root);
+        dev::k_sum_vec<T, dev::kSumReduceScatter, COLS, VEC><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P,
+                                                                                                  n, blk, root, e0);
     else
-        dev::k_sum_vec<T, dev::kSumReduce, COLS><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, ncol,
-                                                                                      blk_vec, root);
+        dev::k_sum_vec<T, dev::kSumReduce, COLS, VEC><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, n,
+                                                                                           blk, root, e0);
     CUDA_TRY(cudaGetLastError());
     return BINE_SUCCESS;
+}
+
+// Sums of elements [e0, e0 + n) of every row (`in` and, except for
+// reduce_scatter, `out` point at element e0).
+template <typename T, bool VEC>
+int launch_sum_range(bine_comm_t c, int mode, const char* in, long long ist, char* out, long long ost, long long n,
+                     long long blk, int root, long long e0) {
+    const int P = c->P;
+    const long long ncol = (n * (long long)sizeof(T) + 15) / 16;
+    // Tiles of 64 columns (4 row groups), or 256 (one group) below
+    // P = 16; narrower while a call would have fewer than two tiles
+    // per SM.  Measured on B200 at 4 MiB per rank (GB/s, old rule ->
+    // 64 columns): P = 16: 6406 -> 7084; 64: 5726 -> 6194; 256: 5716
+    // -> 6347; 1024: 5751 -> 6316.
+    // Below 32 columns a tile has more row groups than that (16 or
+    // 32); only for P of at least two rows per group.
+    int cols = P < 16 ? 256 : 64;
+    while (ncol / cols < 2LL * std::max(1, c->num_sms) &&
+           (cols > 32 || (cols > dev::kSumCols && P >= 2 * (2 * dev::kThreads / cols))))
+        cols /= 2;
+    switch (cols) {
+    case 256: return launch_sum_cols<T, 256, VEC>(c, mode, in, ist, out, ost, P, n, blk, root, e0);
+    case 128: return launch_sum_cols<T, 128, VEC>(c, mode, in, ist, out, ost, P, n, blk, root, e0);
+    case 64: return launch_sum_cols<T, 64, VEC>(c, mode, in, ist, out, ost, P, n, blk, root, e0);
+    case 32: return launch_sum_cols<T, 32, VEC>(c, mode, in, ist, out, ost, P, n, blk, root, e0);
+    case 16: return launch_sum_cols<T, 16, VEC>(c, mode, in, ist, out, ost, P, n, blk, root, e0);
+    default: return launch_sum_cols<T, 8, VEC>(c, mode, in, ist, out, ost, P, n, blk, root, e0);
+    }
 }
 
 template <typename T>
 int launch_sum(bine_comm_t c, int mode, const char* in, long long ist, char* out, long long ost, long long elems,
                long long blk, int root) {
-    const int P = c->P;
     const long long es = sizeof(T);
     const bool vec = aligned16(in) && aligned16(out) && ist % 16 == 0 && ost % 16 == 0 &&
                      (mode != dev::kSumReduceScatter || (blk * es) % 16 == 0);
-    long long done = 0;
-    if (vec) {
-        const long long ncol = elems * es / 16;
-        if (ncol > 0) {
-            const long long blk_vec = mode == dev::kSumReduceScatter ? blk * es / 16 : 0;
-            // Tiles of 64 columns (4 row groups), or 256 (one group) below
-            // P = 16; narrower while a call would have fewer than two tiles
-            // per SM.  Measured on B200 at 4 MiB per rank (GB/s, old rule ->
-            // 64 columns): P = 16: 6406 -> 7084; 64: 5726 -> 6194; 256: 5716
-            // -> 6347; 1024: 5751 -> 6316.
-            // Below 32 columns a tile has more row groups than that (16 or
-            // 32); only for P of at least two rows per group.
-            int cols = P < 16 ? 256 : 64;
-            while (ncol / cols < 2LL * std::max(1, c->num_sms) &&
-                   (cols > 32 || (cols > dev::kSumCols && P >= 2 * (2 * dev::kThreads / cols))))
-                cols /= 2;
-            int rc;
-            switch (cols) {
-            case 256: rc = launch_sum_cols<T, 256>(c, mode, in, ist, out, ost, P, ncol, blk_vec, root); break;
-            case 128: rc = launch_sum_cols<T, 128>(c, mode, in, ist, out, ost, P, ncol, blk_vec, root); break;
-            case 64: rc = launch_sum_cols<T, 64>(c, mode, in, ist, out, ost, P, ncol, blk_vec, root); break;
-            case 32: rc = launch_sum_cols<T, 32>(c, mode, in, ist, out, ost, P, ncol, blk_vec, root); break;
-            case 16: rc = launch_sum_cols<T, 16>(c, mode, in, ist, out, ost, P, ncol, blk_vec, root); break;
-            default: rc = launch_sum_cols<T, 8>(c, mode, in, ist, out, ost, P, ncol, blk_vec, root); break;
-            }
-            if (rc) return rc;
-            done = ncol * 16 / es;
-        }
+    const long long done = vec ? elems * es / 16 * (16 / es) : 0;
+    if (done > 0) {
+        int rc = launch_sum_range<T, true>(c, mode, in, ist, out, ost, done, blk, root, 0);
+        if (rc) return rc;
     }
     const long long rest = elems - done;
-    if (rest > 0) {
-        unsigned g = grid_for(c, rest);
+    if (rest == 0) return BINE_SUCCESS;
+    if constexpr (sizeof(T) == 1) {
+        const unsigned g = grid_for(c, rest);
         if (mode == dev::kSumAllreduce)
-            dev::k_sum_scalar<T, dev::kSumAllreduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, done, rest, blk, root);
+            dev::k_sum_scalar<T, dev::kSumAllreduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, c->P, done, rest, blk, root);
         else if (mode == dev::kSumReduceScatter)
-            dev::k_sum_scalar<T, dev::kSumReduceScatter><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, done, rest, blk, root);
+            dev::k_sum_scalar<T, dev::kSumReduceScatter><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, c->P, done, rest, blk, root);
         else
-            dev::k_sum_scalar<T, dev::kSumReduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, P, done, rest, blk, root);
+            dev::k_sum_scalar<T, dev::kSumReduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, c->P, done, rest, blk, root);
+        CUDA_TRY(cudaGetLastError());
+        return BINE_SUCCESS;
+    } else {
+        const long long off = done * es;
+        return launch_sum_range<T, false>(c, mode, in + off, ist, mode == dev::kSumReduceScatter ? out : out + off,
+                                          ost, rest, blk, root, done);
     }
-    CUDA_TRY(cudaGetLastError());
-    return BINE_SUCCESS;
 }
 
 int launch_sum_dt(bine_comm_t c, int dt, int mode, const char* in, long long ist, char* out, long long ost,

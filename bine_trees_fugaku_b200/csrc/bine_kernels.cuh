@@ -161,45 +161,58 @@ __device__ __forceinline__ uint4 vadd(uint4 a, uint4 b) {
 // ------------------------------------------------------- fused reductions
 enum SumMode { kSumAllreduce = 0, kSumReduceScatter = 1, kSumReduce = 2 };
 
-// Column sums over 16-byte vector columns.  A block owns tiles of COLS
-// vector columns at a time; its 256 threads form 256/COLS row groups that
-// split the P rows of a tile (group g sums rows [g*P/G, (g+1)*P/G) of its
-// lane's column, 8 loads in flight per thread), the partial sums meet in
-// shared memory, and all threads then store the result rows.  The host
-// picks COLS (64 columns and 4 row groups; one group below P = 16; narrower
-// tiles for calls too small to give every SM two tiles) and launches one
-// block per tile up to 64 blocks per SM, beyond which blocks walk the tiles
-// grid-stride.  `ncol` vector columns per input row; reduce_scatter: `blk`
-// vector columns per destination rank.
+// Column sums.  A block owns tiles of COLS lane vectors at a time; its 256
+// threads form 256/COLS row groups that split the P rows of a tile (group g
+// sums rows [g*P/G, (g+1)*P/G) of its lane's vector, 8 loads in flight per
+// thread), the partial sums meet in shared memory, and all threads then
+// store the result rows.  The host picks COLS (64 vectors and 4 row groups;
+// one group below P = 16; narrower tiles for calls too small to give every
+// SM two tiles) and launches one block per tile up to 64 blocks per SM,
+// beyond which blocks walk the tiles grid-stride.
+//
+// The call covers elements [0, n) of rows that start at `in` and `out`;
+// reduce_scatter: `blk` elements per destination rank, and `in` is element
+// `e0` of the row.  VEC: lane vectors of 16 contiguous, aligned bytes (n and
+// blk are whole vectors).  Otherwise strided ones (ld_strided, COLS elements
+// apart), for rows off the 16-byte grid and for the last partial vector:
+// the loop over the rows is the same, with four loads of 4 bytes in the
+// place of one of 16.  They replaced one thread per element with its P rows
+// in a chain (int32 allreduce, us per call): P = 96 at 262,147 elements per
+// rank 47.7 -> 39.3 (37.3 at 262,144, on the grid), P = 256 at 1,048,577
+// 509 -> 381, P = 300 at 777 int64 28.3 -> 8.1, P = 500 at 1 15.0 -> 7.3.
 constexpr int kSumCols = 8;  // the narrowest tile (32 row groups)
 
-template <typename T, int MODE, int COLS>
+template <typename T, int MODE, int COLS, bool VEC>
 __global__ void __launch_bounds__(kThreads) k_sum_vec(const char* __restrict__ in, long long in_stride,
                                                       char* __restrict__ out, long long out_stride, int P,
-                                                      long long ncol, long long blk, int root) {
+                                                      long long n, long long blk, int root, long long e0) {
     using A = typename AccOf<T>::type;
     constexpr int G = kThreads / COLS;
+    constexpr int L = 16 / sizeof(T);
     __shared__ Lanes<T, A> part[G][COLS];
     __shared__ uint4 res[COLS];
     const int lane = threadIdx.x % COLS, grp = threadIdx.x / COLS;
     const int per = (P + G - 1) / G;
     const int r0 = min(P, grp * per), r1 = min(P, r0 + per);
-    const long long ntiles = (ncol + COLS - 1) / COLS;
+    const long long ntiles = (n + COLS * L - 1) / (COLS * L);
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long col = tile * COLS + lane;
+        // The lane's vector: first element, and how many of its elements exist.
+        const long long e = tile * (COLS * L) + (VEC ? lane * L : lane);
+        const int have = VEC ? (e < n ? L : 0) : (int)max(0ll, min((long long)L, (n - e + COLS - 1) / COLS));
+        const auto ld = [&](const char* p) { return VEC ? ld_stream(p) : ld_strided<T, COLS>(p, have); };
         Lanes<T, A> acc;
         acc.zero();
-        if (col < ncol) {
-            const char* p = in + col * 16;
+        if (have > 0) {
+            const char* p = in + e * (long long)sizeof(T);
             int r = r0;
             for (; r + 8 <= r1; r += 8) {
                 uint4 v[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) v[u] = ld_stream(p + (long long)(r + u) * in_stride);
+                for (int u = 0; u < 8; u++) v[u] = ld(p + (long long)(r + u) * in_stride);
 #pragma unroll
                 for (int u = 0; u < 8; u++) acc.add(v[u]);
             }
-            for (; r < r1; r++) acc.add(ld_stream(p + (long long)r * in_stride));
+            for (; r < r1; r++) acc.add(ld(p + (long long)r * in_stride));
         }
         if (G > 1) {
             part[grp][lane] = acc;
@@ -216,17 +229,30 @@ __global__ void __launch_bounds__(kThreads) k_sum_vec(const char* __restrict__ i
         } else {
             res[lane] = acc.pack();
         }
-        if (col < ncol) {
+        if (have > 0) {
             const uint4 v = res[lane];
+            const auto st = [&](char* q) {
+                if (VEC) st_stream(q, v);
+                else st_strided<T, COLS>(q, v, have);
+            };
             if (MODE == kSumAllreduce) {
-                char* q = out + col * 16;
-                for (int d = grp; d < P; d += G) st_stream(q + (long long)d * out_stride, v);
+                char* q = out + e * (long long)sizeof(T);
+                for (int d = grp; d < P; d += G) st(q + (long long)d * out_stride);
             } else if (grp == 0) {
-                if (MODE == kSumReduceScatter) {
-                    const long long owner = col / blk;
-                    st_stream(out + owner * out_stride + (col - owner * blk) * 16, v);
+                if (MODE == kSumReduce) {
+                    st(out + (long long)root * out_stride + e * (long long)sizeof(T));
+                } else if (VEC) {
+                    const long long owner = (e0 + e) / blk;
+                    st(out + owner * out_stride + (e0 + e - owner * blk) * (long long)sizeof(T));
                 } else {
-                    st_stream(out + (long long)root * out_stride + col * 16, v);
+                    const T* t = reinterpret_cast<const T*>(&v);
+#pragma unroll
+                    for (int i = 0; i < L; i++) {
+                        if (i < have) {
+                            const long long x = e0 + e + (long long)i * COLS, owner = x / blk;
+                            __stcs(reinterpret_cast<T*>(out + owner * out_stride) + (x - owner * blk), t[i]);
+                        }
+                    }
                 }
             }
         }
@@ -234,8 +260,10 @@ __global__ void __launch_bounds__(kThreads) k_sum_vec(const char* __restrict__ i
     }
 }
 
-// Element-wise fallback for unaligned layouts and tails: elements
-// [e0, e0 + n) of every row.  reduce_scatter: `blk` elements per rank.
+// Sums of 1-byte elements off the 16-byte grid, elements [e0, e0 + n) of
+// every row, one per thread: a strided lane vector would take 16 loads of
+// one byte each (int8 allreduce at P = 96, 262,147 elements per rank: 20.7 us
+// here, 33.3 us strided).  reduce_scatter: `blk` elements per rank.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kThreads) k_sum_scalar(const char* __restrict__ in, long long in_stride,
                                                          char* __restrict__ out, long long out_stride, int P,

@@ -106,3 +106,33 @@ def test_exact_order_reduce_matches_the_oracle(P, count, root):
     x = values((P, count), np.float32, P)
     want, _ = port.run("reduce", x, count, root=root)
     assert same_bits(call("reduce", x, count, root=root)[root], want[root])
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64, np.int8, np.float64])
+@pytest.mark.parametrize("coll", ["allreduce", "reduce", "reduce_scatter"])
+@pytest.mark.parametrize("P,count,shift,pad", [
+    (2, 1, 0, 0), (3, 5, 1, 0), (7, 1025, 0, 0), (15, 4099, 1, 1), (16, 33, 0, 0), (33, 257, 0, 0), (97, 1031, 0, 2), (200, 3, 0, 0),
+    (64, 2047, 0, 1), (520, 13, 0, 0)])
+def test_sums_off_the_grid(coll, P, count, shift, pad, dtype):
+    """Whole-number sums (FAST order for float64), with ragged tails on rows
+    that are and are not on the 16-byte grid."""
+    si, _ = buffer_counts(coll, count, P)
+    x = values((P, si), np.int32 if dtype == np.float64 else dtype, P * 7 + count).astype(dtype)
+    want = expected(coll, x, P, count, 0)
+    got = call(coll, x, count, shift, pad, order="fast")
+    rows = [0] if coll == "reduce" else slice(None)
+    assert np.array_equal(got[rows], want[rows])
+
+
+@pytest.mark.parametrize("P,count", [(33, 1027), (200, 65)])
+def test_fast_float_sums_off_the_grid(P, count):
+    """FP64 accumulation, one rounding: within half an ulp of the FP64 sum
+    and that sum's own P 2^-52 sum|x|."""
+    x = values((P, count), np.float32, P)
+    want = x.astype(np.float64).sum(0)
+    got = call("allreduce", x, count, order="fast")
+    bound = np.abs(want) * 2.0 ** -24 + P * 2.0 ** -52 * np.abs(x).astype(np.float64).sum(0)
+    assert np.all(np.abs(got - want) <= bound)
+    # A last partial vector on rows that are on the grid: same bound.
+    got = call("allreduce", x, count, pad=4 - count % 4, order="fast")
+    assert np.all(np.abs(got - want) <= bound)
