@@ -1569,12 +1569,78 @@ int launch_tree(bine_comm_t c, const DevTrees& d, const char* in, long long ist,
     return BINE_SUCCESS;
 }
 
-int launch_copy(bine_comm_t c, int mode, const char* in, long long ist, char* out, long long ost, long long unit,
-                int root, int es) {
-    dev::CopyArgs a{in, ist, out, ost, c->P, root, unit, 1};
-    long long pairs = mode == dev::kCopyAlltoall ? (long long)c->P * c->P : (mode == dev::kCopyBcast ? 1 : c->P);
-    if (unit == 0) return BINE_SUCCESS;
-    const bool vec = aligned16(in) && aligned16(out) && ist % 16 == 0 && ost % 16 == 0 && unit % 16 == 0;
+template <typename U>
+int launch_copy_units(bine_comm_t c, int mode, dev::CopyArgs a) {
+    const long long sms = std::max(1, c->num_sms);
+    const bool spread = mode == dev::kCopyAllgather || mode == dev::kCopyBcast;
+    const long long pairs = mode == dev::kCopyAlltoall ? (long long)a.P * a.P : (mode == dev::kCopyBcast ? 1 : a.P);
+    const long long nu = a.unit / (long long)sizeof(U), units = pairs * nu;
+    const long long fill = 2LL * dev::kThreads * sms;
+    a.by_ranks = dev::FastDiv(a.P, pairs);
+    if constexpr (sizeof(U) == 4 || sizeof(U) == 8) {
+        // Broadcasts off the 16-byte grid, from 8 MiB written: below, and
+        // for a few rows, the staging costs more than it gains (us, k_copy
+        // / k_spread: allgather at P = 300, 33 int32 6.3 / 7.5; bcast at
+        // P = 8, 1,000,003 int32 8.5 / 8.9).
+        if (spread && a.P >= 16 && a.P * pairs * a.unit >= (8ll << 20)) {
+            dev::SpreadArgs sa;
+            sa.in = mode == dev::kCopyBcast ? a.in + (long long)a.root * a.in_stride : a.in;
+            sa.in_stride = a.in_stride;
+            sa.out = a.out;
+            sa.out_stride = a.out_stride;
+            sa.P = a.P;
+            sa.skip = mode == dev::kCopyBcast ? a.root : -1;
+            sa.n = pairs * a.unit;
+            sa.unit = mode == dev::kCopyBcast || a.in_stride == a.unit ? sa.n : a.unit;
+            sa.ntiles = (sa.n + dev::kSpreadTile - 1) / dev::kSpreadTile;
+            sa.groups = (int)std::max<long long>(1, std::min<long long>((a.P + 7) / 8, (dev::kSpreadItems * sms + sa.ntiles - 1) / sa.ntiles));
+            sa.by_tiles = dev::FastDiv(sa.ntiles, sa.ntiles * sa.groups);
+            sa.by_unit = dev::FastDiv(sa.unit / (long long)sizeof(U), sa.n / (long long)sizeof(U));
+            if (sa.ntiles * sa.groups <= INT32_MAX) {
+                dev::k_spread<U><<<(unsigned)(sa.ntiles * sa.groups), dev::kSpreadThreads, 0, c->stream>>>(sa);
+                CUDA_TRY(cudaGetLastError());
+                return BINE_SUCCESS;
+            }
+        }
+    }
+    if (!spread && nu >= dev::kCopyBlockMin) {
+        // Realigned vectors for 4-byte elements from 1 KiB per block and for
+        // narrower ones from 256 bytes; elements otherwise (us, elements /
+        // realigned: alltoall at P = 256 with 516-byte blocks 25 / 45, with
+        // 1,028-byte blocks 50 / 47; P = 16 with 65,537 int64 46 / 50).
+        const bool shift = sizeof(U) <= 4 && a.unit >= (sizeof(U) == 4 ? 1024 : 256);
+        long long blocks;
+        if (shift) {
+            a.chunks = (a.unit / 16 + dev::kShiftVecs - 1) / dev::kShiftVecs;
+            a.groups = pairs * a.chunks;
+            blocks = (a.groups + dev::kThreads / 32 - 1) / (dev::kThreads / 32);
+        } else {
+            constexpr long long kE = sizeof(U) == 16 ? 4 : 8;  // elements per thread, as in k_copy_blocks
+            while ((1 << a.tp_log2) < dev::kThreads && kE << a.tp_log2 < nu) a.tp_log2++;
+            a.chunks = (nu + (kE << a.tp_log2) - 1) / (kE << a.tp_log2);
+            a.groups = pairs * a.chunks;
+            blocks = ((a.groups << a.tp_log2) + dev::kThreads - 1) / dev::kThreads;
+        }
+        a.by_chunks = dev::FastDiv(a.chunks, a.groups);
+        const unsigned g = (unsigned)std::max(1LL, std::min(blocks, sms * 64));
+#define BINE_COPY(M)                                                                                     \
+    case dev::M:                                                                                         \
+        if constexpr (sizeof(U) <= 4)                                                                    \
+            if (shift) {                                                                                 \
+                dev::k_copy_shift<dev::M, U><<<g, dev::kThreads, 0, c->stream>>>(a);                     \
+                break;                                                                                   \
+            }                                                                                            \
+        dev::k_copy_blocks<dev::M, U><<<g, dev::kThreads, 0, c->stream>>>(a);                            \
+        break;
+        switch (mode) {
+            BINE_COPY(kCopyAlltoall)
+            BINE_COPY(kCopyScatter)
+            BINE_COPY(kCopyGather)
+        }
+#undef BINE_COPY
+        CUDA_TRY(cudaGetLastError());
+        return BINE_SUCCESS;
+    }
     // Allgather and bcast store every source vector to P rows.  A call whose
     // source units would give fewer than half the SMs a block leaves most
     // of the GPU idle: its rows are then split over threads, enough groups
@@ -1583,40 +1649,76 @@ int launch_copy(bine_comm_t c, int mode, const char* in, long long ist, char* ou
     // on B200 (int64, us): bcast P = 1024 at 8 KiB per rank 69.7 -> 4.4,
     // allgather P = 1024 at 32 B 69.8 -> 8.3; allgather P = 1024 at 512 B
     // (128 blocks) 78 unsplit, 95 split in 3.
-    const long long units = pairs * (vec ? unit / 16 : unit / es);
-    const long long fill = 2LL * dev::kThreads * std::max(1, c->num_sms);
-    if ((mode == dev::kCopyAllgather || mode == dev::kCopyBcast) && 4 * units < fill)
+    a.dgroups = 1;
+    if (spread && 4 * units < fill)
         a.dgroups = (int)std::max<long long>(1, std::min<long long>(std::max(1, c->P / 8), (fill + units - 1) / units));
-    if (vec) {
-        unsigned g = grid_for(c, pairs * (unit / 16) * a.dgroups);
+    if (!spread) {
+        const unsigned g = grid_for(c, units);
+        const bool narrow = units < (1ll << 31);
+#define BINE_COPY(M)                                                                                     \
+    case dev::M:                                                                                         \
+        if (narrow) dev::k_copy_small<dev::M, U, unsigned><<<g, dev::kThreads, 0, c->stream>>>(a);       \
+        else dev::k_copy_small<dev::M, U, long long><<<g, dev::kThreads, 0, c->stream>>>(a);             \
+        break;
         switch (mode) {
-        case dev::kCopyAllgather: dev::k_copy_vec<dev::kCopyAllgather><<<g, dev::kThreads, 0, c->stream>>>(a); break;
-        case dev::kCopyBcast: dev::k_copy_vec<dev::kCopyBcast><<<g, dev::kThreads, 0, c->stream>>>(a); break;
-        case dev::kCopyAlltoall: dev::k_copy_vec<dev::kCopyAlltoall><<<g, dev::kThreads, 0, c->stream>>>(a); break;
-        case dev::kCopyScatter: dev::k_copy_vec<dev::kCopyScatter><<<g, dev::kThreads, 0, c->stream>>>(a); break;
-        case dev::kCopyGather: dev::k_copy_vec<dev::kCopyGather><<<g, dev::kThreads, 0, c->stream>>>(a); break;
+            BINE_COPY(kCopyAlltoall)
+            BINE_COPY(kCopyScatter)
+            BINE_COPY(kCopyGather)
         }
-    } else {
-        unsigned g = grid_for(c, pairs * (unit / es) * a.dgroups);
-#define BINE_COPY_SCALAR(U)                                                                                          \
-    switch (mode) {                                                                                                  \
-    case dev::kCopyAllgather: dev::k_copy_scalar<dev::kCopyAllgather, U><<<g, dev::kThreads, 0, c->stream>>>(a); break; \
-    case dev::kCopyBcast: dev::k_copy_scalar<dev::kCopyBcast, U><<<g, dev::kThreads, 0, c->stream>>>(a); break;         \
-    case dev::kCopyAlltoall: dev::k_copy_scalar<dev::kCopyAlltoall, U><<<g, dev::kThreads, 0, c->stream>>>(a); break;   \
-    case dev::kCopyScatter: dev::k_copy_scalar<dev::kCopyScatter, U><<<g, dev::kThreads, 0, c->stream>>>(a); break;     \
-    case dev::kCopyGather: dev::k_copy_scalar<dev::kCopyGather, U><<<g, dev::kThreads, 0, c->stream>>>(a); break;       \
+#undef BINE_COPY
+        CUDA_TRY(cudaGetLastError());
+        return BINE_SUCCESS;
     }
-        if (es == 8 && ((uintptr_t)in | (uintptr_t)out | ist | ost | unit) % 8 == 0) {
-            BINE_COPY_SCALAR(uint64_t)
-        } else if (es >= 4 && ((uintptr_t)in | (uintptr_t)out | ist | ost | unit) % 4 == 0) {
-            BINE_COPY_SCALAR(uint32_t)
-        } else {
-            BINE_COPY_SCALAR(uint8_t)
+    // Broadcasts on the 16-byte grid: a block writes P rows (or its share of
+    // them), so with 256 threads per block the SMs that got one block more
+    // finish a whole block's time after the others.  Smaller blocks where
+    // that costs more than 7 % of the time, except for calls small enough
+    // for the block launches to count; and for bcast, whose rows are one run
+    // each, two vectors per thread from one block of 256 per SM.  us on
+    // B200, 256 threads -> this rule: allgather at P = 96, 32 KiB 55.6 -> 52.4,
+    // P = 300, 2 KiB 45.3 -> 31.6, P = 512, 512 B 29.3 -> 25.1; bcast at P = 16,
+    // 4 MiB 14.8 -> 13.0, P = 384, 2 MiB 140 -> 131, P = 512, 128 KiB 16.5 ->
+    // 14.6; kept at 256: allgather at P = 128, 32 KiB 90.1 (93.0 with 64),
+    // bcast at P = 256, 512 KiB 22.5 (23.9 with 32).
+    int threads = dev::kThreads, E = 1;
+    if (sizeof(U) == 16 && a.P * pairs * a.unit >= (32ll << 20)) {
+        const long long full = (units + dev::kThreads - 1) / dev::kThreads, turns = (full + sms - 1) / sms;
+        if (full > sms && mode == dev::kCopyBcast) {
+            threads = 32;
+            E = 2;
+        } else if (full > sms && 100 * full < 93 * turns * sms) {
+            threads = 64;
+        } else if (4 * full < 3 * sms) {
+            threads = 32;
         }
-#undef BINE_COPY_SCALAR
     }
+    const long long per = E == 1 ? units : (units + 32 * E - 1) / (32 * E) * 32;  // threads, as in the kernel
+    const long long blocks = (per * a.dgroups + threads - 1) / threads;
+    const unsigned g = (unsigned)std::max(1LL, std::min(blocks, 16LL * sms * (dev::kThreads / threads)));
+    if (mode == dev::kCopyAllgather) dev::k_copy_rows<dev::kCopyAllgather, U, 1><<<g, threads, 0, c->stream>>>(a);
+    else if (E == 2) dev::k_copy_rows<dev::kCopyBcast, U, 2><<<g, threads, 0, c->stream>>>(a);
+    else dev::k_copy_rows<dev::kCopyBcast, U, 1><<<g, threads, 0, c->stream>>>(a);
     CUDA_TRY(cudaGetLastError());
     return BINE_SUCCESS;
+}
+
+int launch_copy(bine_comm_t c, int mode, const char* in, long long ist, char* out, long long ost, long long unit,
+                int root) {
+    if (unit == 0) return BINE_SUCCESS;
+    dev::CopyArgs a{};
+    a.in = in;
+    a.in_stride = ist;
+    a.out = out;
+    a.out_stride = ost;
+    a.P = c->P;
+    a.root = root;
+    a.unit = unit;
+    const uintptr_t bits = (uintptr_t)in | (uintptr_t)out | (uintptr_t)ist | (uintptr_t)ost | (uintptr_t)unit;
+    if (bits % 16 == 0) return launch_copy_units<uint4>(c, mode, a);
+    if (bits % 8 == 0) return launch_copy_units<uint64_t>(c, mode, a);
+    if (bits % 4 == 0) return launch_copy_units<uint32_t>(c, mode, a);
+    if (bits % 2 == 0) return launch_copy_units<uint16_t>(c, mode, a);
+    return launch_copy_units<uint8_t>(c, mode, a);
 }
 
 // ------------------------------------------------------------ step engine
@@ -1862,11 +1964,11 @@ int run_collective(bine_comm_t c, int coll, const void* sendbuf, void* recvbuf, 
         return launch_sum_dt(c, dt, mode, in, ist, out, ost, se, count, root);
     }
     switch (coll) {
-    case kAllgather: return launch_copy(c, dev::kCopyAllgather, in, ist, out, ost, count * es, root, es);
-    case kBcast: return launch_copy(c, dev::kCopyBcast, out, ost, out, ost, count * es, root, es);
-    case kAlltoall: return launch_copy(c, dev::kCopyAlltoall, in, ist, out, ost, count * es, root, es);
-    case kScatter: return launch_copy(c, dev::kCopyScatter, in, ist, out, ost, count * es, root, es);
-    case kGather: return launch_copy(c, dev::kCopyGather, in, ist, out, ost, count * es, root, es);
+    case kAllgather: return launch_copy(c, dev::kCopyAllgather, in, ist, out, ost, count * es, root);
+    case kBcast: return launch_copy(c, dev::kCopyBcast, out, ost, out, ost, count * es, root);
+    case kAlltoall: return launch_copy(c, dev::kCopyAlltoall, in, ist, out, ost, count * es, root);
+    case kScatter: return launch_copy(c, dev::kCopyScatter, in, ist, out, ost, count * es, root);
+    case kGather: return launch_copy(c, dev::kCopyGather, in, ist, out, ost, count * es, root);
     }
     return fail(BINE_ERR_ARG, "unknown collective");
 }

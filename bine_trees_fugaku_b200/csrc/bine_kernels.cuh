@@ -75,12 +75,21 @@ __device__ __forceinline__ T ld_stream_elem(const void* p) {
         unsigned r;
         asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(r) : "l"(p));
         memcpy(&v, &r, 4);
+    } else if constexpr (sizeof(T) == 2) {
+        unsigned short r;
+        asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(r) : "l"(p));
+        memcpy(&v, &r, 2);
     } else {
         unsigned r;
         asm volatile("ld.global.nc.L1::no_allocate.u8 %0, [%1];" : "=r"(r) : "l"(p));
         v = (T)r;
     }
     return v;
+}
+__device__ __forceinline__ uint4 ld_unit(const uint4* p) { return ld_stream(p); }
+template <typename U>
+__device__ __forceinline__ U ld_unit(const U* p) {
+    return __ldg(p);  // through L1: neighbouring runs off the 128-byte grid share sectors
 }
 template <typename T, int STEP>
 __device__ __forceinline__ uint4 ld_strided(const char* p, int n) {
@@ -90,6 +99,11 @@ __device__ __forceinline__ uint4 ld_strided(const char* p, int n) {
 #pragma unroll
     for (int i = 0; i < N; i++) t[i] = i < n ? ld_stream_elem<T>(p + i * STEP * (int)sizeof(T)) : (T)0;
     return raw;
+}
+template <typename T>
+__device__ __forceinline__ void st_cs(T* p, T v) {
+    if constexpr (sizeof(T) == 16) st_stream(p, v);
+    else __stcs(p, v);
 }
 template <typename T, int STEP>
 __device__ __forceinline__ void st_strided(char* p, uint4 raw, int n) {
@@ -958,6 +972,27 @@ __global__ void __launch_bounds__(kThreads) k_tree_strided(const char* __restric
 // ----------------------------------------------------------------- copies
 enum CopyMode { kCopyAllgather = 0, kCopyBcast = 1, kCopyAlltoall = 2, kCopyScatter = 3, kCopyGather = 4 };
 
+// Division of n < 2^31 by a fixed d as one multiplication and a shift
+// (Granlund and Montgomery, "Division by invariant integers using
+// multiplication": with l = ceil(log2 d) and m = floor(2^(31+l) / d) + 1,
+// floor(n / d) = floor(n * m / 2^(31+l))).  Larger n divide directly (mul 0).
+struct FastDiv {
+    long long d = 1;
+    unsigned mul = 0;
+    int shift = 0;
+    FastDiv() = default;
+    FastDiv(long long divisor, long long max_n) : d(divisor) {
+        if (max_n >= (1ll << 31) || divisor >= (1ll << 31)) return;
+        int l = 0;
+        while ((1ll << l) < divisor) l++;
+        shift = 31 + l;
+        mul = (unsigned)((1ull << shift) / (unsigned long long)divisor + 1);
+    }
+    __device__ __forceinline__ long long operator()(long long n) const {
+        return mul ? (long long)(((unsigned long long)(unsigned)n * mul) >> shift) : n / d;
+    }
+};
+
 // A copy collective is a set of "pairs" (source row piece, destination row
 // pieces) of `unit` bytes each; unit = one rank's block.
 struct CopyArgs {
@@ -967,97 +1002,294 @@ struct CopyArgs {
     long long out_stride;
     int P;
     int root;
-    long long unit;  // bytes per block
-    int dgroups;     // allgather / bcast: destination groups per source vector (>= 1)
+    long long unit;    // bytes per block
+    int dgroups;       // k_copy, allgather / bcast: destination groups per source element (>= 1)
+    // k_copy_blocks, k_copy_shift: a pair is cut into `chunks` pieces.
+    long long groups;  // pairs * chunks
+    long long chunks;
+    int tp_log2;       // k_copy_blocks: log2 of the threads per piece
+    FastDiv by_chunks, by_ranks;
 };
 
+// Source of pair `i` (alltoall: block `to` of row `from`), and its
+// destination in the collectives that have one.
 template <int MODE>
-__device__ __forceinline__ long long copy_pairs(const CopyArgs& a) {
-    if (MODE == kCopyAlltoall) return (long long)a.P * a.P;
-    if (MODE == kCopyBcast) return 1;
-    return a.P;
-}
-
-// Source of pair `i` and its destinations (first and count; bcast and
-// allgather broadcast one load to several rows).
-template <int MODE>
-__device__ __forceinline__ const char* copy_src(const CopyArgs& a, long long i) {
+__device__ __forceinline__ const char* copy_src(const CopyArgs& a, long long i, long long from, long long to) {
     if (MODE == kCopyAllgather) return a.in + i * a.in_stride;
     if (MODE == kCopyBcast) return a.in + (long long)a.root * a.in_stride;
-    if (MODE == kCopyAlltoall) {
-        long long src = i / a.P, dst = i % a.P;  // block dst of row src
-        return a.in + src * a.in_stride + dst * a.unit;
-    }
+    if (MODE == kCopyAlltoall) return a.in + from * a.in_stride + to * a.unit;
     if (MODE == kCopyScatter) return a.in + (long long)a.root * a.in_stride + i * a.unit;
     return a.in + i * a.in_stride;  // gather
 }
 template <int MODE>
-__device__ __forceinline__ int copy_ndst(const CopyArgs& a) {
-    if (MODE == kCopyAllgather) return a.P;
-    if (MODE == kCopyBcast) return a.P;
-    return 1;
-}
-// Allgather and bcast calls with few source vectors split each vector's
-// destinations over `dgroups` threads (each loads the vector and stores to
-// its share of the rows), so that small calls still fill the GPU.
-template <int MODE>
-__device__ __forceinline__ int copy_groups(const CopyArgs& a) {
-    return (MODE == kCopyAllgather || MODE == kCopyBcast) ? max(1, a.dgroups) : 1;
-}
-template <int MODE>
-__device__ __forceinline__ char* copy_dst(const CopyArgs& a, long long i, int d) {
-    if (MODE == kCopyAllgather) return a.out + (long long)d * a.out_stride + i * a.unit;
-    if (MODE == kCopyBcast) return d == a.root ? nullptr : a.out + (long long)d * a.out_stride;
-    if (MODE == kCopyAlltoall) {
-        long long src = i / a.P, dst = i % a.P;
-        return a.out + dst * a.out_stride + src * a.unit;
-    }
+__device__ __forceinline__ char* copy_dst(const CopyArgs& a, long long i, long long from, long long to) {
+    if (MODE == kCopyAlltoall) return a.out + to * a.out_stride + from * a.unit;
     if (MODE == kCopyScatter) return a.out + i * a.out_stride;
     return a.out + (long long)a.root * a.out_stride + i * a.unit;  // gather
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kThreads) k_copy_vec(CopyArgs a) {
-    const long long nvec = a.unit / 16;
+// The element type U of these kernels is the widest whose size divides every
+// address, stride and block length of the call (uint4 when all are on the
+// 16-byte grid).
+//
+template <typename U>
+__device__ __forceinline__ void st_unit(U* p, U v) {
+    if constexpr (sizeof(U) == 16) st_stream(p, v);
+    else *p = v;  // partial sectors: the neighbours' parts meet in L2 (bcast, P = 8, 1,000,003 int32: 8.5 us, 12.8 with .cs)
+}
+
+// The broadcasting collectives (each element to P rows): E elements per
+// thread, 32 apart, over the elements of all blocks in order.  Calls with few
+// source elements split each element's destinations over `dgroups` threads
+// (each loads it and stores to its share of the rows), so that small calls
+// still fill the GPU.
+template <int MODE, typename U, int E>
+__global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_copy_rows(CopyArgs a) {
+    const long long nu = a.unit / (long long)sizeof(U);
     const long long step = (long long)gridDim.x * blockDim.x;
-    if constexpr (MODE == kCopyAllgather || MODE == kCopyBcast) {
-        const int G = copy_groups<MODE>(a);
-        const long long per = copy_pairs<MODE>(a) * nvec, total = per * G;
-        for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += step) {
-            const long long gi = G == 1 ? 0 : w / per, r = w - gi * per;
-            const long long i = r / nvec, j = r - i * nvec;
-            const uint4 v = ld_stream(copy_src<MODE>(a, i) + j * 16);
-            const int nd = copy_ndst<MODE>(a);
-            const int d0 = (int)(nd * gi / G), d1 = (int)(nd * (gi + 1) / G);
-            for (int d = d0; d < d1; d++) {
-                char* q = copy_dst<MODE>(a, i, d);
-                if (q) st_stream(q + j * 16, v);
-            }
+    const int G = a.dgroups;
+    const long long n = (MODE == kCopyBcast ? 1 : a.P) * nu;
+    const long long per = E == 1 ? n : (n + 32 * E - 1) / (32 * E) * 32, total = per * G;  // threads: whole warps
+    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += step) {
+        const long long gi = G == 1 ? 0 : w / per, r = w - gi * per;
+        const long long x0 = E == 1 ? r : (r - (r & 31)) * E + (r & 31);
+        U v[E];
+#pragma unroll
+        for (int u = 0; u < E; u++) {
+            const long long x = x0 + 32 * u;
+            if (E > 1 && x >= n) continue;  // the last warp's
+            const long long i = MODE == kCopyBcast ? 0 : x / nu;
+            v[u] = ld_unit(reinterpret_cast<const U*>(copy_src<MODE>(a, i, 0, 0)) + (x - i * nu));
         }
-    } else {  // one destination per source vector
-        const long long total = copy_pairs<MODE>(a) * nvec;
-        for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += step) {
-            const long long i = w / nvec, j = w - (w / nvec) * nvec;
-            st_stream(copy_dst<MODE>(a, i, 0) + j * 16, ld_stream(copy_src<MODE>(a, i) + j * 16));
+        const int d0 = (int)(a.P * gi / G), d1 = (int)(a.P * (gi + 1) / G);
+        char* q = a.out + (long long)d0 * a.out_stride + x0 * (long long)sizeof(U);
+        // Unrolled for element stores only: 16-byte stores run ahead of the
+        // other blocks' (allgather, P = 128, 32 KiB: 90.1 us, 93.4 unrolled).
+#pragma unroll(sizeof(U) == 16 ? 1 : 4)
+        for (int d = d0; d < d1; d++, q += a.out_stride) {
+            if (MODE == kCopyBcast && d == a.root) continue;
+#pragma unroll
+            for (int u = 0; u < E; u++)
+                if (E == 1 || x0 + 32 * u < n) st_unit(reinterpret_cast<U*>(q) + 32 * u, v[u]);
         }
     }
 }
 
-template <int MODE, typename U>
-__global__ void __launch_bounds__(kThreads) k_copy_scalar(CopyArgs a) {
-    const long long nu = a.unit / (long long)sizeof(U);
-    const int G = copy_groups<MODE>(a);
-    const long long per = copy_pairs<MODE>(a) * nu, total = per * G;
+// Blocks of fewer than kCopyBlockMin elements with one destination: four
+// elements per thread and round, over the elements of all blocks in order
+// (I: the index type, 32 bits where the element count allows).
+template <int MODE, typename U, typename I>
+__global__ void __launch_bounds__(kThreads) k_copy_small(CopyArgs a) {
+    const I nu = (I)(a.unit / (long long)sizeof(U)), P = (I)a.P;
+    const long long total = (MODE == kCopyAlltoall ? (long long)a.P * a.P : a.P) * (a.unit / (long long)sizeof(U));
     const long long step = (long long)gridDim.x * blockDim.x;
-    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += step) {
-        const long long gi = G == 1 ? 0 : w / per, r = w - gi * per;
-        const long long i = r / nu, j = r - i * nu;
-        const U v = *(const U*)(copy_src<MODE>(a, i) + j * sizeof(U));
-        const int nd = copy_ndst<MODE>(a);
-        const int d0 = (int)(nd * gi / G), d1 = (int)(nd * (gi + 1) / G);
-        for (int d = d0; d < d1; d++) {
-            char* q = copy_dst<MODE>(a, i, d);
-            if (q) *(U*)(q + j * sizeof(U)) = v;
+    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += 4 * step) {
+        U v[4];
+        U* q[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            if (w + x * step >= total) continue;
+            const I e = (I)(w + x * step), i = e / nu, j = e - i * nu;
+            const I from = MODE == kCopyAlltoall ? i / P : 0, to = i - from * P;
+            v[x] = ld_unit(reinterpret_cast<const U*>(copy_src<MODE>(a, i, from, to)) + j);
+            q[x] = reinterpret_cast<U*>(copy_dst<MODE>(a, i, from, to)) + j;
+        }
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+            if (w + x * step < total) st_unit(q[x], v[x]);
+    }
+}
+
+// Blocks of at least kCopyBlockMin elements with one destination (alltoall,
+// scatter, gather): a group of 2^tp_log2 threads moves a piece of up to E
+// elements per thread, 2^tp_log2 apart, so that a warp's accesses are
+// contiguous runs, E loads are in flight before the stores, and the block
+// numbers are divided out once per thread instead of once per element.
+// Bound by HBM.  Against k_copy (us, B200): alltoall at P = 64 with 64 KiB
+// blocks 89 -> 82, P = 256 with 516-byte blocks 38 -> 25.
+constexpr int kCopyBlockMin = 16;
+template <int MODE, typename U>
+__global__ void __launch_bounds__(kThreads) k_copy_blocks(CopyArgs a) {
+    constexpr int E = sizeof(U) == 16 ? 4 : 8;
+    const int tp = 1 << a.tp_log2;
+    const long long nu = a.unit / (long long)sizeof(U);
+    const long long step = (long long)gridDim.x * blockDim.x >> a.tp_log2;
+    const int t = threadIdx.x & (tp - 1);
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> a.tp_log2; w < a.groups; w += step) {
+        const long long i = a.chunks == 1 ? w : a.by_chunks(w);
+        const long long first = (w - i * a.chunks) * (tp * E) + t;
+        const long long from = MODE == kCopyAlltoall ? a.by_ranks(i) : 0, to = i - from * a.P;
+        const int have = (int)min((long long)E, (nu - first + tp - 1) >> a.tp_log2);
+        const U* src = reinterpret_cast<const U*>(copy_src<MODE>(a, i, from, to)) + first;
+        U* dst = reinterpret_cast<U*>(copy_dst<MODE>(a, i, from, to)) + first;
+        U v[E];
+#pragma unroll
+        for (int u = 0; u < E; u++)
+            if (u < have) v[u] = ld_unit(src + u * tp);
+#pragma unroll
+        for (int u = 0; u < E; u++)
+            if (u < have) st_cs(dst + u * tp, v[u]);
+    }
+}
+
+// Allgather and bcast off the 16-byte grid: every row receives the same
+// sequence of n bytes, but the rows start at different offsets within 16
+// bytes.  A block stages one tile of the sequence in shared memory once per
+// such offset (16 / sizeof(U) copies, each shifted by one element more), so
+// that the body of every row's tile is one bulk copy (cp.async.bulk, 16-byte
+// aligned on both sides) from the copy that matches the row; the up to 30
+// bytes before and after it are element stores.  Rows are split into groups
+// to give the GPU about kSpreadItems blocks per SM.
+//
+// Bound by HBM writes: element stores off the grid leave two partial
+// sectors per 128 bytes.  Measured on B200 (us): bcast at P = 96,
+// 1,000,001 int32 116 -> 73, allgather at P = 41, 20,001 floats 40.1 ->
+// 28.5.  Rows on the grid need no staging and stay with k_copy (allgather
+// at P = 96, 32 KiB: 52.4 there, 58 here).
+constexpr int kSpreadThreads = 128;
+constexpr int kSpreadTile = 4096;  // bytes of the sequence per block
+constexpr int kSpreadItems = 20;
+struct SpreadArgs {
+    const char* in;
+    long long in_stride;
+    char* out;
+    long long out_stride;
+    int P, skip;      // skip: the row that already holds the sequence, or -1
+    long long n;      // bytes of the sequence
+    long long unit;   // bytes of one contiguous source piece (n: one piece)
+    int groups;       // row groups
+    long long ntiles;
+    FastDiv by_tiles, by_unit;  // by_unit: elements of type U
+};
+
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+                 : "memory");
+}
+
+template <typename U>
+__global__ void __launch_bounds__(kSpreadThreads) k_spread(const SpreadArgs a) {
+    constexpr int kVar = 16 / sizeof(U);
+    constexpr int kBatch = 8;
+    __shared__ __align__(128) char sbuf[kVar][kSpreadTile];
+    const long long g = a.by_tiles(blockIdx.x), x0 = (blockIdx.x - g * a.ntiles) * kSpreadTile;
+    const int n = (int)min((long long)kSpreadTile, a.n - x0), nu = n / (int)sizeof(U);
+    const long long u0 = x0 / (long long)sizeof(U), pu = a.unit / (long long)sizeof(U);
+    for (int b = threadIdx.x; b < nu; b += kBatch * kSpreadThreads) {
+        U v[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int x = b + u * kSpreadThreads;
+            if (x < nu) {
+                const long long e = u0 + x, i = a.unit == a.n ? 0 : a.by_unit(e);
+                v[u] = ld_unit(reinterpret_cast<const U*>(a.in + i * a.in_stride) + (e - i * pu));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            const int x = b + u * kSpreadThreads;
+            if (x < nu) {
+#pragma unroll
+                for (int s = 0; s < kVar; s++)
+                    if (x >= s) *reinterpret_cast<U*>(sbuf[s] + (x - s) * (int)sizeof(U)) = v[u];
+            }
+        }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the bulk copies read what this thread wrote
+    __syncthreads();
+    const uint32_t sb = (uint32_t)__cvta_generic_to_shared(sbuf);
+    const int d0 = (int)(a.P * g / a.groups), d1 = (int)(a.P * (g + 1) / a.groups);
+    for (int d = d0 + threadIdx.x; d < d1; d += kSpreadThreads) {
+        if (d == a.skip) continue;
+        char* dst = a.out + (long long)d * a.out_stride + x0;
+        const int head = min(n, (int)(16 - ((uintptr_t)dst & 15)) & 15), body = (n - head) & ~15;
+        if (body > 0) bulk_store(dst + head, sb + head / (int)sizeof(U) * kSpreadTile, body);
+        for (int x = 0; x < head; x += (int)sizeof(U)) *reinterpret_cast<U*>(dst + x) = *reinterpret_cast<U*>(sbuf[0] + x);
+        for (int x = head + body; x < n; x += (int)sizeof(U))
+            *reinterpret_cast<U*>(dst + x) = *reinterpret_cast<U*>(sbuf[0] + x);
+    }
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory is read before the block ends
+}
+
+// Blocks whose source and destination do not share a 16-byte grid (alltoall,
+// scatter, gather): 16-byte loads on the source's grid, realigned in
+// registers, 16-byte stores on the destination's.  A warp copies kShiftVecs
+// destination vectors of one block; a lane's vector is cut from the aligned
+// source vector it loaded and the next one, which lane + 1 loaded (lane 31:
+// lane 0's of the next 32).  Only source vectors that lie inside the block
+// are read, so up to 31 bytes at a block's start and 47 at its end are
+// copied as elements of type U.
+//
+// Bound by HBM: whole-sector stores, where element stores off the grid leave
+// two partial sectors per 128 bytes.  Measured on B200 (us, one element per
+// thread -> this kernel): alltoall at P = 64 with blocks of 10,001 int32 158
+// -> 64, of 10,001 bytes 153 -> 18.8; P = 128 with 2,052-byte blocks 37.4 ->
+// 16.7.
+constexpr int kShiftVecs = 128;  // destination vectors per warp
+template <int MODE, typename U>
+__global__ void __launch_bounds__(kThreads) k_copy_shift(CopyArgs a) {
+    constexpr int kE = kShiftVecs / 32;
+    const int lane = threadIdx.x & 31;
+    const long long step = (long long)gridDim.x * (kThreads / 32);
+    for (long long w = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); w < a.groups; w += step) {
+        const long long i = a.chunks == 1 ? w : a.by_chunks(w);
+        const long long chunk = w - i * a.chunks;
+        const long long from = MODE == kCopyAlltoall ? a.by_ranks(i) : 0, to = i - from * a.P;
+        const char* src = copy_src<MODE>(a, i, from, to);
+        char* dst = copy_dst<MODE>(a, i, from, to);
+        // Destination vectors [0, nvec) start `head` bytes into the block;
+        // source vector k of its own grid starts at src + head - off + 16k,
+        // and destination vector k takes bytes off.. of vectors k and k + 1.
+        const int head = (int)(16 - ((uintptr_t)dst & 15)) & 15;
+        const int off = (int)((uintptr_t)(src + head) & 15);
+        const long long nvec = (a.unit - head) / 16;
+        const long long k0 = head >= off ? 0 : 1, k1 = max(k0, min(nvec, (a.unit - head + off) / 16 - 1));
+        const char* s = src + head - off;
+        char* d = dst + head;
+        const long long kb = chunk * (32 * kE) + lane;
+        uint4 v[kE + 1];
+#pragma unroll
+        for (int j = 0; j <= kE; j++) {
+            const long long k = kb + 32 * j;
+            v[j] = make_uint4(0, 0, 0, 0);
+            if (k >= k0 && k <= k1 && (j < kE || lane == 0)) v[j] = ld_stream(s + 16 * k);
+        }
+        uint4 t = v[0];  // the vectors one lane up, of this 32 and of the next
+        auto up = [&](uint4 x) {
+            const int from = (lane + 1) & 31;
+            return make_uint4(__shfl_sync(0xffffffffu, x.x, from), __shfl_sync(0xffffffffu, x.y, from),
+                              __shfl_sync(0xffffffffu, x.z, from), __shfl_sync(0xffffffffu, x.w, from));
+        };
+        t = up(v[0]);
+        const int q = off >> 2, b = (off & 3) * 8;
+#pragma unroll
+        for (int j = 0; j < kE; j++) {
+            const uint4 tn = up(v[j + 1]);
+            const uint4 n = lane == 31 ? tn : t;
+            t = tn;
+            uint32_t x[8] = {v[j].x, v[j].y, v[j].z, v[j].w, n.x, n.y, n.z, n.w};
+            if (q & 2) {
+#pragma unroll
+                for (int z = 0; z < 6; z++) x[z] = x[z + 2];
+            }
+            if (q & 1) {
+#pragma unroll
+                for (int z = 0; z < 5; z++) x[z] = x[z + 1];
+            }
+            const long long k = kb + 32 * j;
+            if (k >= k0 && k < k1)
+                st_stream(d + 16 * k,
+                          make_uint4(__funnelshift_r(x[0], x[1], b), __funnelshift_r(x[1], x[2], b),
+                                     __funnelshift_r(x[2], x[3], b), __funnelshift_r(x[3], x[4], b)));
+        }
+        if (chunk == 0) {
+            const int n = (int)min(a.unit, head + 16 * k0) / (int)sizeof(U);
+            for (int e = lane; e < n; e += 32) reinterpret_cast<U*>(dst)[e] = reinterpret_cast<const U*>(src)[e];
+        }
+        if (chunk == a.chunks - 1) {
+            const long long from = min(a.unit, head + 16 * k1) / (long long)sizeof(U), n = a.unit / (long long)sizeof(U);
+            for (long long e = from + lane; e < n; e += 32) reinterpret_cast<U*>(dst)[e] = reinterpret_cast<const U*>(src)[e];
         }
     }
 }

@@ -31,7 +31,7 @@ def call(coll, x, count, shift=0, pad=0, variant=None, lanes=0, order="reference
     buffers that start `shift` elements after a 16-byte boundary; checks the
     guards and the padding."""
     P = x.shape[0]
-    si, so = buffer_counts(coll, count, P)
+    si, so = x.shape[1], buffer_counts(coll, count, P)[1]
     td = torch.from_numpy(x[:1, :1]).dtype
     comm = bine.Comm(P)
     if variant:
@@ -136,3 +136,58 @@ def test_fast_float_sums_off_the_grid(P, count):
     # A last partial vector on rows that are on the grid: same bound.
     got = call("allreduce", x, count, pad=4 - count % 4, order="fast")
     assert np.all(np.abs(got - want) <= bound)
+
+
+@pytest.mark.parametrize("dtype", [np.int8, np.int32, np.int64])
+@pytest.mark.parametrize("coll", ["alltoall", "scatter", "gather"])
+@pytest.mark.parametrize("P,count,shift,pad", [
+    (2, 1, 0, 0), (5, 3, 1, 0), (7, 16, 1, 0), (16, 17, 0, 1), (33, 64, 0, 0), (9, 255, 3, 0), (6, 257, 1, 2), (12, 1021, 0, 0),
+    (8, 2047, 1, 0), (8, 2049, 3, 5), (5, 4096, 0, 0), (4, 10_001, 1, 1), (64, 40, 0, 4)])
+def test_block_copies_off_the_grid(coll, P, count, shift, pad, dtype):
+    """Blocks from one element to several pieces of a warp, at every kind of
+    offset between source and destination."""
+    root = P // 2
+    si, _ = buffer_counts(coll, count, P)
+    x = values((P, si), dtype, P + count)
+    want = expected(coll, x, P, count, root)
+    got = call(coll, x, count, shift, pad, root=root)
+    rows = [root] if coll == "gather" else slice(None)
+    assert np.array_equal(got[rows], want[rows])
+
+
+@pytest.mark.parametrize("dtype", [np.int8, np.int32, np.int64])
+@pytest.mark.parametrize("coll,P,count,shift,pad", [
+    ("bcast", 3, 1, 0, 0), ("bcast", 16, 131_073, 1, 0), ("bcast", 17, 130_003, 0, 1), ("bcast", 40, 65_540, 1, 0),
+    ("bcast", 200, 11_003, 0, 0), ("bcast", 33, 4096, 0, 0),
+    ("allgather", 3, 5, 1, 0), ("allgather", 48, 1001, 0, 0), ("allgather", 48, 1001, 1, 3), ("allgather", 130, 129, 0, 0),
+    ("allgather", 16, 8200, 0, 1), ("allgather", 37, 64, 0, 0)])
+def test_broadcasts_off_the_grid(coll, P, count, shift, pad, dtype):
+    """Below and above the size from which tiles are staged for bulk copies;
+    rows at every offset within 16 bytes, packed and padded sources."""
+    root = P // 3
+    si, _ = buffer_counts("allreduce" if coll == "bcast" else coll, count, P)
+    x = values((P, si), dtype, P + count)
+    want = expected(coll, x, P, count, root)
+    assert np.array_equal(call(coll, x, count, shift, pad, root=root), want)
+
+
+@pytest.mark.parametrize("coll,P,count", [
+    ("bcast", 56, 4 * 37_889), ("bcast", 56, 4 * (37_889 + 33)), ("bcast", 56, 4 * 50_000 + 4), ("bcast", 300, 4 * 20_001),
+    ("bcast", 70, 4 * 30_003), ("allgather", 65, 4 * 600), ("allgather", 40, 4 * 1400), ("allgather", 300, 4 * 37), ("allgather", 96, 4 * 333)])
+def test_large_broadcasts_on_the_grid(coll, P, count):
+    """From 32 MiB written: one warp per block with one and two vectors per
+    thread, 64 and 256 threads; the last warp partly filled."""
+    x = torch.randint(-1000, 1001, (P, count), dtype=torch.int32, device="cuda", generator=torch.Generator("cuda").manual_seed(P))
+    so = count * (P if coll == "allgather" else 1)
+    out = torch.full((P * so + 2 * GUARD,), 77, dtype=torch.int32, device="cuda")
+    y = out[GUARD:GUARD + P * so].view(P, so)
+    comm = bine.Comm(P)
+    comm.set_stream(torch.cuda.current_stream())
+    if coll == "bcast":
+        y[3] = x[3]
+    comm.run(coll, x, y, count, bine.INT32, 3)
+    comm.synchronize()
+    want = x.reshape(-1) if coll == "allgather" else x[3]
+    assert bool((y == want).all())
+    assert bool((out[:GUARD] == 77).all()) and bool((out[GUARD + P * so:] == 77).all())
+    comm.close()
