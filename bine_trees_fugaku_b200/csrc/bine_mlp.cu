@@ -4,9 +4,9 @@
 //
 // Shape: in -> H -> H -> H -> out (3 hidden layers of width H, GELU after
 // each hidden layer, exact erf form).  All dimensions are multiples of 16.
-// GEMMs use warp-level tensor-core tiles (wmma 16x16x16, bf16 in, fp32
-// accumulate); at this model size (H = 256) the network is bound by launch
-// latency, not by tensor throughput.
+// GEMMs use warp-level tensor-core tiles (mma m16n8k16, bf16 in, fp32
+// accumulate); at this model size (H = 256) the network is bound by latency,
+// not by tensor throughput.
 //
 //   forward:  pre_l = act_{l-1} W_l^T + b_l (fp32), act_l = bf16(gelu(pre_l))
 //   loss:     masked mean squared error of the output against targets
@@ -16,9 +16,9 @@
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-#include <mma.h>
 
 #include <cmath>
+#include <cstring>
 #include <memory>
 #include <random>
 #include <string>
@@ -29,7 +29,6 @@
 namespace {
 
 using bf16 = __nv_bfloat16;
-using namespace nvcuda;
 
 thread_local std::string g_mlp_err;
 
@@ -44,55 +43,6 @@ int mfail(int code, const std::string& m) {
         if (e_ != cudaSuccess) return mfail(BINE_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// C[M x N] (fp32, row-major, ldc) = A[M x K] * B[K x N]; A and B bf16 in the
-// given layouts.  Block: 4 warps, 64 x 64 tile; warp: 32 x 32 (2 x 2 tiles).
-template <typename ALayout, typename BLayout>
-__global__ void __launch_bounds__(128) k_gemm(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B,
-                                              int ldb, float* __restrict__ C, int ldc, int M, int N, int K) {
-    const int warp = threadIdx.x / 32;
-    const int wm = blockIdx.y * 64 + (warp / 2) * 32;
-    const int wn = blockIdx.x * 64 + (warp % 2) * 32;
-    wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++) wmma::fill_fragment(acc[i][j], 0.0f);
-    for (int k = 0; k < K; k += 16) {
-        wmma::fragment<wmma::matrix_a, 16, 16, 16, bf16, ALayout> a[2];
-        wmma::fragment<wmma::matrix_b, 16, 16, 16, bf16, BLayout> b[2];
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int r = wm + i * 16;
-            if (r < M) {
-                const bf16* p = std::is_same<ALayout, wmma::row_major>::value ? A + (size_t)r * lda + k
-                                                                              : A + (size_t)k * lda + r;
-                wmma::load_matrix_sync(a[i], p, lda);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int c = wn + j * 16;
-            if (c < N) {
-                const bf16* p = std::is_same<BLayout, wmma::row_major>::value ? B + (size_t)k * ldb + c
-                                                                              : B + (size_t)c * ldb + k;
-                wmma::load_matrix_sync(b[j], p, ldb);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-            for (int j = 0; j < 2; j++)
-                if (wm + i * 16 < M && wn + j * 16 < N) wmma::mma_sync(acc[i][j], a[i], b[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-            if (wm + i * 16 < M && wn + j * 16 < N)
-                wmma::store_matrix_sync(C + (size_t)(wm + i * 16) * ldc + wn + j * 16, acc[i][j], ldc,
-                                        wmma::mem_row_major);
-}
-
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float x) {
     const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
@@ -100,50 +50,294 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return cdf + x * pdf;
 }
 
-// pre += bias; act = bf16(gelu(pre)) (hidden) or out = pre (last layer).
-__global__ void k_bias_act(float* pre, const float* bias, bf16* act, int M, int N, int hidden) {
-    const long long n = (long long)M * N;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float v = pre[i] + bias[i % N];
-        pre[i] = v;
-        if (hidden) act[i] = __float2bfloat16(gelu(v));
+// ------------------------------------------------- layered forward/backward
+// Every GEMM of the layered path is a few hundred rows and columns: bound by
+// the latency of its operand loads and of the launches between dependent
+// stages, not by tensor throughput.  So a block owns one 32 x 32 tile (four
+// warps of 16 x 16), requests its operands for 2 * kStageK steps of the
+// reduction at once (cp.async, double-buffered beyond that), and what
+// follows a GEMM runs in its epilogue on the accumulators: bias and GELU,
+// loss and output gradient, GELU' of the backward pass, bias gradients (from
+// the staged tiles).  One stage per dependent step remains: a prepare kernel,
+// 4 forward, 4 backward (the weight gradient of a layer beside the next
+// layer's input gradient).  Each accumulator adds its k-steps of 16 in
+// ascending order.
+//
+// B200, 256 rows, 16 -> 256 -> 256 -> 256 -> 144, host call included, against
+// one launch per GEMM (64 x 64 tiles, operands loaded step by step), bias,
+// loss, GELU' and column sum, with the mask counted on the host: gradients
+// 559 -> 124 us (about 60 of them the copy of 690 KB to the host and its
+// fresh pages), training step 400 -> 73, forward 57 -> 22.
+constexpr int kTile = 32;      // rows and columns of a block's tile
+constexpr int kStageK = 128;   // reduction steps per buffer
+constexpr int kGemmThreads = 128;
+constexpr int kPitchK = kStageK + 8;  // operand stored [row][k]: 16-byte rows fall on distinct banks
+constexpr int kPitchT = kTile + 8;    // operand stored [k][row]
+
+struct GemmSmem {
+    // One buffer holds a [kTile][kPitchK] or a [kStageK][kPitchT] tile.
+    static constexpr int kElems = kStageK * kPitchT > kTile * kPitchK ? kStageK * kPitchT : kTile * kPitchK;
+    __align__(128) bf16 a[2][kElems];
+    __align__(128) bf16 b[2][kElems];
+};
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
+                 : "memory");
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix_x4(uint32_t* r, const void* smem) {
+    const uint32_t p = (uint32_t)__cvta_generic_to_shared(smem);
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(p)
+                     : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(p)
+                     : "memory");
+}
+__device__ __forceinline__ void mma_bf16_16816(float* d, const uint32_t* a, const uint32_t* b) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// Requests k-steps [k0, k0 + kn) of a tile's 32 rows from `row0` of an
+// operand: stored [row][k] (ld elements per row), or [k][row] when T.  Rows
+// from `rows` on are not requested (their results are not used); all
+// dimensions are multiples of 16, so every request is 16 aligned bytes.
+template <bool T>
+__device__ __forceinline__ void gemm_request(bf16* smem, const bf16* __restrict__ g, int ld, int row0, int rows,
+                                             int k0, int kn) {
+    const int nr = min(kTile, rows - row0);
+    if (!T) {
+        const int per = kn / 8;  // 16-byte pieces per row
+        for (int i = threadIdx.x; i < nr * per; i += kGemmThreads) {
+            const int r = i / per, c = i - r * per;
+            cp_async16(smem + r * kPitchK + c * 8, g + (size_t)(row0 + r) * ld + k0 + c * 8);
+        }
+    } else {
+        const int per = nr / 8;
+        for (int i = threadIdx.x; i < kn * per; i += kGemmThreads) {
+            const int k = i / per, c = i - k * per;
+            cp_async16(smem + k * kPitchT + c * 8, g + (size_t)(k0 + k) * ld + row0 + c * 8);
+        }
     }
 }
 
-// Masked MSE: d = mask * (y - t); loss += d^2; grad = bf16(2 d / count).
-__global__ void k_loss(const float* y, const float* t, const float* mask, bf16* grad, float* loss, int M, int N,
-                       float inv_count) {
-    __shared__ float red[256];
-    float acc = 0.f;
-    const long long n = (long long)M * N;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float d = mask[i] * (y[i] - t[i]);
-        acc += d * d;
-        grad[i] = __float2bfloat16(2.0f * d * inv_count);
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+// acc (two 16 x 8 fragments of the warp's 16 x 16) = A[row0.., :] B[:, col0..]
+// over K.  A is stored [M][K] (lda), or [K][M] when TA; B [N][K] (ldb), or
+// [K][N] when TB.  `each(buffer, steps)` sees every staged A tile.
+template <bool TA, bool TB, typename Each>
+__device__ __forceinline__ void gemm_tile(GemmSmem& S, float (&acc)[2][4], const bf16* __restrict__ A, int lda,
+                                          const bf16* __restrict__ B, int ldb, int row0, int col0, int M, int N,
+                                          int K, const Each& each) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
+    const bool active = row0 + wm < M && col0 + wn < N;
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[h][i] = 0.f;
+    const int stages = (K + kStageK - 1) / kStageK;
+    auto request = [&](int s) {
+        if (s < stages) {
+            const int k0 = s * kStageK, kn = min(kStageK, K - k0);
+            gemm_request<TA>(S.a[s & 1], A, lda, row0, M, k0, kn);
+            gemm_request<TB>(S.b[s & 1], B, ldb, col0, N, k0, kn);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    request(0);
+    request(1);
+    for (int s = 0; s < stages; s++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
+        const int kn = min(kStageK, K - s * kStageK);
+        const bf16* sa = S.a[s & 1];
+        const bf16* sb = S.b[s & 1];
+        if (active) {
+            // ldmatrix: lanes 8q .. 8q + 7 address the rows of matrix q.
+            const int q = lane >> 3, r = lane & 7;
+#pragma unroll 4
+            for (int k = 0; k < kn; k += 16) {
+                uint32_t a[4], b[4];
+                if (!TA) ldmatrix_x4<false>(a, sa + (wm + (q & 1) * 8 + r) * kPitchK + k + (q >> 1) * 8);
+                else ldmatrix_x4<true>(a, sa + (k + (q >> 1) * 8 + r) * kPitchT + wm + (q & 1) * 8);
+                if (!TB) ldmatrix_x4<false>(b, sb + (wn + (q >> 1) * 8 + r) * kPitchK + k + (q & 1) * 8);
+                else ldmatrix_x4<true>(b, sb + (k + (q & 1) * 8 + r) * kPitchT + wn + (q >> 1) * 8);
+                mma_bf16_16816(acc[0], a, b);
+                mma_bf16_16816(acc[1], a, b + 2);
+            }
+        }
+        each(sa, kn);
+        __syncthreads();  // the buffer is free for the request after next
+        request(s + 2);
     }
-    if (threadIdx.x == 0) atomicAdd(loss, red[0] * inv_count);
 }
 
-// d_pre = bf16(d_act * gelu'(pre)).
-__global__ void k_gelu_back(const float* dact, const float* pre, bf16* dpre, int M, int N) {
-    const long long n = (long long)M * N;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        dpre[i] = __float2bfloat16(dact[i] * gelu_grad(pre[i]));
+// Calls f(row, column, value 0, value 1) for the warp's accumulators: two
+// adjacent columns at a time.
+template <typename F>
+__device__ __forceinline__ void gemm_each(const float (&acc)[2][4], int row0, int col0, int M, int N, const F& f) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r = row0 + (warp >> 1) * 16 + (lane >> 2), c = col0 + (warp & 1) * 16 + (lane & 3) * 2;
+    if (row0 + (warp >> 1) * 16 >= M || col0 + (warp & 1) * 16 >= N) return;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        f(r, c + 8 * h, acc[h][0], acc[h][1]);
+        f(r + 8, c + 8 * h, acc[h][2], acc[h][3]);
+    }
 }
 
-// db[j] = sum_i d_pre[i][j] (fp32 accumulation of the bf16 gradients).
-__global__ void k_colsum(const bf16* g, float* db, int M, int N) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    float s = 0.f;
-    for (int i = 0; i < M; i++) s += __bfloat162float(g[(size_t)i * N + j]);
-    db[j] = s;
+// x in bf16, and per block the valid (mask != 0) targets it counted.
+constexpr int kPrepBlocks = 64;
+__global__ void __launch_bounds__(256) k_prepare(const float* __restrict__ x, bf16* __restrict__ xb, long long n,
+                                                 const float* __restrict__ mask, long long m, int* counts) {
+    const long long step = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (long long i = first; i < n; i += step) xb[i] = __float2bfloat16(x[i]);
+    if (!mask) return;
+    int c = 0;
+    for (long long i = first; i < m; i += step) c += mask[i] != 0.f;
+    __shared__ int warp_sum[8];
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) c += warp_sum[w];
+        counts[blockIdx.x] = c;
+    }
+}
+
+// One layer: pre = in W^T + bias.  Hidden: pre and act = bf16(gelu(pre)).
+// Output (act null): y = pre, and with targets the masked MSE (d = mask (y -
+// t); loss = mean of d^2 over the valid entries, one partial sum per block;
+// grad = bf16(2 d / count)).
+struct ForwardArgs {
+    const bf16 *in, *w;
+    const float* bias;
+    float* pre;
+    bf16* act;
+    float* y;
+    const float *t, *mask;
+    const int* counts;
+    float* losses;
+    bf16* grad;
+    int M, N, K;
+};
+__global__ void __launch_bounds__(kGemmThreads) k_forward(const ForwardArgs a) {
+    __shared__ GemmSmem S;
+    float acc[2][4];
+    const int row0 = blockIdx.y * kTile, col0 = blockIdx.x * kTile;
+    gemm_tile<false, false>(S, acc, a.in, a.K, a.w, a.K, row0, col0, a.M, a.N, a.K, [](const bf16*, int) {});
+    if (a.act) {
+        gemm_each(acc, row0, col0, a.M, a.N, [&](int r, int c, float v0, float v1) {
+            const size_t i = (size_t)r * a.N + c;
+            v0 += a.bias[c];
+            v1 += a.bias[c + 1];
+            *reinterpret_cast<float2*>(a.pre + i) = make_float2(v0, v1);
+            *reinterpret_cast<__nv_bfloat162*>(a.act + i) = __floats2bfloat162_rn(gelu(v0), gelu(v1));
+        });
+        return;
+    }
+    float inv = 0.f, sum = 0.f;
+    if (a.t) {
+        __shared__ int total[2];
+        if (threadIdx.x < kPrepBlocks) {
+            const int c = __reduce_add_sync(0xffffffffu, a.counts[threadIdx.x]);
+            if ((threadIdx.x & 31) == 0) total[threadIdx.x >> 5] = c;
+        }
+        __syncthreads();
+        const int count = total[0] + total[1];
+        inv = count > 0 ? (float)(1.0 / count) : 0.f;
+    }
+    gemm_each(acc, row0, col0, a.M, a.N, [&](int r, int c, float v0, float v1) {
+        const size_t i = (size_t)r * a.N + c;
+        v0 += a.bias[c];
+        v1 += a.bias[c + 1];
+        if (a.y) {  // the caller's array: any float alignment
+            a.y[i] = v0;
+            a.y[i + 1] = v1;
+        }
+        if (a.t) {
+            const float d0 = a.mask[i] * (v0 - a.t[i]), d1 = a.mask[i + 1] * (v1 - a.t[i + 1]);
+            sum += d0 * d0;
+            sum += d1 * d1;
+            *reinterpret_cast<__nv_bfloat162*>(a.grad + i) = __floats2bfloat162_rn(2.0f * d0 * inv, 2.0f * d1 * inv);
+        }
+    });
+    if (a.t) {
+        __shared__ float part[kGemmThreads / 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            a.losses[blockIdx.y * gridDim.x + blockIdx.x] = (part[0] + part[1] + part[2] + part[3]) * inv;
+    }
+}
+
+// One backward stage from a layer's gradient `g` [n][N].  Blocks below
+// nx * ny: the gradient of the layer below, bf16((g W) gelu'(pre)) [n][K].
+// The others: dW = g^T in [N][K] and, from the staged gradients, db = column
+// sums of g.  The first block also adds up the loss (deterministic).
+struct BackwardArgs {
+    const bf16 *g, *w, *in;
+    const float* pre;
+    bf16* below;
+    float *dw, *db;
+    int n, N, K;
+    int nx, ny;  // tiles of the gradient below (0: first layer)
+    const float* losses;
+    int nlosses;
+    float* loss;
+};
+__global__ void __launch_bounds__(kGemmThreads) k_backward(const BackwardArgs a) {
+    __shared__ GemmSmem S;
+    float acc[2][4];
+    int tile = blockIdx.x;
+    if (tile < a.nx * a.ny) {
+        const int row0 = tile / a.nx * kTile, col0 = tile % a.nx * kTile;
+        gemm_tile<false, true>(S, acc, a.g, a.N, a.w, a.K, row0, col0, a.n, a.K, a.N, [](const bf16*, int) {});
+        gemm_each(acc, row0, col0, a.n, a.K, [&](int r, int c, float v0, float v1) {
+            const size_t i = (size_t)r * a.K + c;
+            const float2 p = *reinterpret_cast<const float2*>(a.pre + i);
+            *reinterpret_cast<__nv_bfloat162*>(a.below + i) =
+                __floats2bfloat162_rn(v0 * gelu_grad(p.x), v1 * gelu_grad(p.y));
+        });
+    } else {
+        tile -= a.nx * a.ny;
+        const int tx = (a.K + kTile - 1) / kTile;
+        const int row0 = tile / tx * kTile, col0 = tile % tx * kTile;
+        const bool sums = col0 == 0;
+        float db = 0.f;  // thread (q, c): column row0 + c of g, rows q mod 4
+        const int c = threadIdx.x & 31, q = threadIdx.x >> 5;
+        gemm_tile<true, true>(S, acc, a.g, a.N, a.in, a.K, row0, col0, a.N, a.K, a.n, [&](const bf16* sg, int kn) {
+            if (sums && row0 + c < a.N)
+                for (int k = q; k < kn; k += 4) db += __bfloat162float(sg[k * kPitchT + c]);
+        });
+        gemm_each(acc, row0, col0, a.N, a.K, [&](int r, int cc, float v0, float v1) {
+            *reinterpret_cast<float2*>(a.dw + (size_t)r * a.K + cc) = make_float2(v0, v1);
+        });
+        if (sums) {
+            __shared__ float part[4][kTile];
+            part[q][c] = db;
+            __syncthreads();
+            if (q == 0 && row0 + c < a.N) a.db[row0 + c] = (part[0][c] + part[1][c]) + (part[2][c] + part[3][c]);
+        }
+    }
+    if (a.losses && blockIdx.x == 0 && threadIdx.x < 32) {
+        float sum = 0.f;
+        for (int i = threadIdx.x; i < a.nlosses; i += 32) sum += a.losses[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (threadIdx.x == 0) *a.loss = sum;
+    }
 }
 
 __global__ void k_to_bf16(const float* x, bf16* y, long long n) {
@@ -195,14 +389,6 @@ struct EnsArgs {
     const float* x;  // [n][din]
     float* y;        // [n][dout], the mean over the models
 };
-
-__device__ __forceinline__ void mma_bf16_16816(float* d, const uint32_t* a, const uint32_t* b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
 
 // One layer for 16 rows: out[16][N] = act[16][K] W^T + bias, then GELU into
 // the next activation buffer (hidden) or fp32 into `outf` (last layer).
@@ -354,13 +540,13 @@ struct bine_mlp_s {
     long long step = 0;
     // Activations for max_batch rows.
     bf16* x = nullptr;           // input, bf16
-    float* pre[4] = {nullptr};   // pre-activations / outputs (fp32)
+    float* pre[3] = {nullptr};   // hidden pre-activations (fp32)
     bf16* act[3] = {nullptr};    // hidden activations (bf16)
-    float* dact = nullptr;       // backprop scratch (fp32)
-    bf16* dpre = nullptr;        // bf16 gradient of the current layer
+    bf16* dpre[2] = {nullptr};   // bf16 gradients of two consecutive layers
+    int* counts = nullptr;       // valid targets per prepare block
+    float* losses = nullptr;     // loss per output tile, then the loss
     float* loss = nullptr;
-    float* t = nullptr;          // targets
-    float* mask = nullptr;
+    float* staged = nullptr;     // pinned host copy of the gradients and the loss
     ~bine_mlp_s() {
         cudaFree(w);
         cudaFree(g);
@@ -370,72 +556,90 @@ struct bine_mlp_s {
         cudaFree(x);
         for (float* p : pre) cudaFree(p);
         for (bf16* p : act) cudaFree(p);
-        cudaFree(dact);
-        cudaFree(dpre);
-        cudaFree(loss);
-        cudaFree(t);
-        cudaFree(mask);
+        for (bf16* p : dpre) cudaFree(p);
+        cudaFree(counts);
+        cudaFree(losses);
+        cudaFreeHost(staged);
     }
 };
 
 namespace {
 
-template <typename AL, typename BL>
-void gemm(const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, int M, int N, int K, cudaStream_t s) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    k_gemm<AL, BL><<<grid, 128, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
+int tiles(int n) { return (n + kTile - 1) / kTile; }
+
+// Rows of the batch (and the targets' mask, for a loss) to the layered path.
+int prepare_batch(bine_mlp_t mlp, const float* d_x, const float* d_mask, int n, cudaStream_t s) {
+    if (!mlp || !d_x || n <= 0 || n > mlp->max_batch || n % 16) return mfail(BINE_ERR_ARG, "batch must be a multiple of 16 within max_batch");
+    k_prepare<<<kPrepBlocks, 256, 0, s>>>(d_x, mlp->x, (long long)n * mlp->din, d_mask, (long long)n * mlp->dout,
+                                          mlp->counts);
+    return BINE_SUCCESS;
 }
 
-// Forward pass of `n` rows already in mlp->x.
-void forward(bine_mlp_t mlp, int n, cudaStream_t s) {
-    const bf16* in = mlp->x;
+// Targets and mask are read by the kernels where they are: device memory (or
+// host memory the device can reach).
+int check_targets(const float* d_t, const float* d_mask) {
+    for (const float* p : {d_t, d_mask}) {
+        cudaPointerAttributes at;
+        if (!p) return mfail(BINE_ERR_ARG, "null targets or mask");
+        MLP_TRY(cudaPointerGetAttributes(&at, p));
+        if (at.type == cudaMemoryTypeUnregistered) return mfail(BINE_ERR_ARG, "targets and mask must be device arrays");
+    }
+    return BINE_SUCCESS;
+}
+
+// Forward pass of the `n` prepared rows: to d_y, or with targets to the
+// output gradient and the loss partials.
+void forward(bine_mlp_t mlp, int n, float* d_y, const float* d_t, const float* d_mask, cudaStream_t s) {
     for (int l = 0; l < mlp->nlayer; l++) {
-        const int K = mlp->in_dim[l], N = mlp->out_dim[l];
-        gemm<wmma::row_major, wmma::col_major>(in, K, mlp->wb + mlp->woff[l], K, mlp->pre[l], N, n, N, K, s);
         const bool hidden = l + 1 < mlp->nlayer;
-        k_bias_act<<<grid1((long long)n * N), 256, 0, s>>>(mlp->pre[l], mlp->w + mlp->boff[l], hidden ? mlp->act[l] : nullptr,
-                                                         n, N, hidden ? 1 : 0);
-        if (hidden) in = mlp->act[l];
+        ForwardArgs a{};
+        a.in = l == 0 ? mlp->x : mlp->act[l - 1];
+        a.w = mlp->wb + mlp->woff[l];
+        a.bias = mlp->w + mlp->boff[l];
+        a.M = n;
+        a.N = mlp->out_dim[l];
+        a.K = mlp->in_dim[l];
+        if (hidden) {
+            a.pre = mlp->pre[l];
+            a.act = mlp->act[l];
+        } else {
+            a.y = d_y;
+            a.t = d_t;
+            a.mask = d_mask;
+            a.counts = mlp->counts;
+            a.losses = mlp->losses;
+            a.grad = mlp->dpre[l & 1];
+        }
+        k_forward<<<dim3(tiles(a.N), tiles(n)), kGemmThreads, 0, s>>>(a);
     }
 }
 
-// Backward pass from the output gradient in mlp->dpre (bf16, n x dout):
-// fills mlp->g with the gradients of every weight and bias.
+// Backward pass: fills mlp->g with the gradients of every weight and bias
+// and *mlp->loss.
 void backward(bine_mlp_t mlp, int n, cudaStream_t s) {
     for (int l = mlp->nlayer - 1; l >= 0; l--) {
-        const int K = mlp->in_dim[l], N = mlp->out_dim[l];
-        const bf16* a_in = l == 0 ? mlp->x : mlp->act[l - 1];
-        // dW = d_pre^T (N x n) * a_in (n x K): fp32 into the gradient arena.
-        gemm<wmma::col_major, wmma::row_major>(mlp->dpre, N, a_in, K, mlp->g + mlp->woff[l], K, N, K, n, s);
-        k_colsum<<<(N + 127) / 128, 128, 0, s>>>(mlp->dpre, mlp->g + mlp->boff[l], n, N);
+        BackwardArgs a{};
+        a.n = n;
+        a.N = mlp->out_dim[l];
+        a.K = mlp->in_dim[l];
+        a.g = mlp->dpre[l & 1];
+        a.w = mlp->wb + mlp->woff[l];
+        a.in = l == 0 ? mlp->x : mlp->act[l - 1];
+        a.dw = mlp->g + mlp->woff[l];
+        a.db = mlp->g + mlp->boff[l];
         if (l > 0) {
-            // d_act_{l-1} = d_pre (n x N) * W (N x K).
-            gemm<wmma::row_major, wmma::row_major>(mlp->dpre, N, mlp->wb + mlp->woff[l], K, mlp->dact, K, n, K, N, s);
-            k_gelu_back<<<grid1((long long)n * K), 256, 0, s>>>(mlp->dact, mlp->pre[l - 1], mlp->dpre, n, K);
+            a.pre = mlp->pre[l - 1];
+            a.below = mlp->dpre[(l - 1) & 1];
+            a.nx = tiles(a.K);
+            a.ny = tiles(n);
         }
+        if (l == mlp->nlayer - 1) {
+            a.losses = mlp->losses;
+            a.nlosses = tiles(mlp->dout) * tiles(n);
+            a.loss = mlp->loss;
+        }
+        k_backward<<<a.nx * a.ny + tiles(a.N) * tiles(a.K), kGemmThreads, 0, s>>>(a);
     }
-}
-
-int load_batch(bine_mlp_t mlp, const float* d_x, int n, cudaStream_t s) {
-    if (!mlp || !d_x || n <= 0 || n > mlp->max_batch || n % 16) return mfail(BINE_ERR_ARG, "batch must be a multiple of 16 within max_batch");
-    k_to_bf16<<<grid1((long long)n * mlp->din), 256, 0, s>>>(d_x, mlp->x, (long long)n * mlp->din);
-    return BINE_SUCCESS;
-}
-
-int loss_and_grad(bine_mlp_t mlp, const float* d_t, const float* d_mask, int n, cudaStream_t s) {
-    MLP_TRY(cudaMemsetAsync(mlp->loss, 0, sizeof(float), s));
-    MLP_TRY(cudaMemcpyAsync(mlp->t, d_t, sizeof(float) * (size_t)n * mlp->dout, cudaMemcpyDeviceToDevice, s));
-    MLP_TRY(cudaMemcpyAsync(mlp->mask, d_mask, sizeof(float) * (size_t)n * mlp->dout, cudaMemcpyDeviceToDevice, s));
-    // Mean over the valid (mask != 0) entries: the caller's mask count.
-    std::vector<float> hm((size_t)n * mlp->dout);
-    MLP_TRY(cudaMemcpyAsync(hm.data(), d_mask, sizeof(float) * hm.size(), cudaMemcpyDeviceToHost, s));
-    MLP_TRY(cudaStreamSynchronize(s));
-    double cnt = 0;
-    for (float q : hm) cnt += q != 0.f;
-    const float inv = cnt > 0 ? (float)(1.0 / cnt) : 0.f;
-    k_loss<<<grid1((long long)n * mlp->dout), 256, 0, s>>>(mlp->pre[mlp->nlayer - 1], mlp->t, mlp->mask, mlp->dpre,
-                                                           mlp->loss, n, mlp->dout, inv);
-    return BINE_SUCCESS;
 }
 
 }  // namespace
@@ -485,14 +689,17 @@ int bine_mlp_create(int in_dim, int hidden, int out_dim, int max_batch, unsigned
     MLP_TRY(cudaMemset(m->v, 0, off * sizeof(float)));
     k_to_bf16<<<grid1(off), 256>>>(m->w, m->wb, (long long)off);
     MLP_TRY(cudaMalloc(&m->x, (size_t)max_batch * in_dim * sizeof(bf16)));
-    for (int l = 0; l < 4; l++) MLP_TRY(cudaMalloc(&m->pre[l], (size_t)max_batch * dims[l + 1] * sizeof(float)));
-    for (int l = 0; l < 3; l++) MLP_TRY(cudaMalloc(&m->act[l], (size_t)max_batch * hidden * sizeof(bf16)));
-    const int wmax = std::max(std::max(in_dim, hidden), out_dim);
-    MLP_TRY(cudaMalloc(&m->dact, (size_t)max_batch * wmax * sizeof(float)));
-    MLP_TRY(cudaMalloc(&m->dpre, (size_t)max_batch * wmax * sizeof(bf16)));
-    MLP_TRY(cudaMalloc(&m->loss, sizeof(float)));
-    MLP_TRY(cudaMalloc(&m->t, (size_t)max_batch * out_dim * sizeof(float)));
-    MLP_TRY(cudaMalloc(&m->mask, (size_t)max_batch * out_dim * sizeof(float)));
+    for (int l = 0; l < 3; l++) {
+        MLP_TRY(cudaMalloc(&m->pre[l], (size_t)max_batch * hidden * sizeof(float)));
+        MLP_TRY(cudaMalloc(&m->act[l], (size_t)max_batch * hidden * sizeof(bf16)));
+    }
+    for (int l = 0; l < 2; l++)
+        MLP_TRY(cudaMalloc(&m->dpre[l], (size_t)max_batch * std::max(hidden, out_dim) * sizeof(bf16)));
+    MLP_TRY(cudaMalloc(&m->counts, kPrepBlocks * sizeof(int)));
+    const size_t nlosses = (size_t)tiles(max_batch) * tiles(out_dim);
+    MLP_TRY(cudaMalloc(&m->losses, (nlosses + 1) * sizeof(float)));
+    m->loss = m->losses + nlosses;
+    MLP_TRY(cudaMallocHost(&m->staged, (off + 1) * sizeof(float)));
     MLP_TRY(cudaDeviceSynchronize());
     *out = m.release();
     return BINE_SUCCESS;
@@ -525,11 +732,10 @@ int bine_mlp_set_params(bine_mlp_t mlp, const float* host) {
 
 int bine_mlp_forward(bine_mlp_t mlp, const float* d_x, int n, float* d_y, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = load_batch(mlp, d_x, n, s);
+    if (!d_y) return mfail(BINE_ERR_ARG, "null output");
+    int rc = prepare_batch(mlp, d_x, nullptr, n, s);
     if (rc) return rc;
-    forward(mlp, n, s);
-    MLP_TRY(cudaMemcpyAsync(d_y, mlp->pre[mlp->nlayer - 1], sizeof(float) * (size_t)n * mlp->dout,
-                            cudaMemcpyDeviceToDevice, s));
+    forward(mlp, n, d_y, nullptr, nullptr, s);
     MLP_TRY(cudaGetLastError());
     return BINE_SUCCESS;
 }
@@ -537,27 +743,30 @@ int bine_mlp_forward(bine_mlp_t mlp, const float* d_x, int n, float* d_y, void* 
 int bine_mlp_gradients(bine_mlp_t mlp, const float* d_x, const float* d_t, const float* d_mask, int n, float* host_grads,
                        float* loss) {
     cudaStream_t s = 0;
-    int rc = load_batch(mlp, d_x, n, s);
+    int rc = check_targets(d_t, d_mask);
+    if (rc == BINE_SUCCESS) rc = prepare_batch(mlp, d_x, d_mask, n, s);
     if (rc) return rc;
-    forward(mlp, n, s);
-    rc = loss_and_grad(mlp, d_t, d_mask, n, s);
-    if (rc) return rc;
+    forward(mlp, n, nullptr, d_t, d_mask, s);
     backward(mlp, n, s);
-    MLP_TRY(cudaStreamSynchronize(s));
-    if (host_grads) MLP_TRY(cudaMemcpy(host_grads, mlp->g, mlp->nparams * sizeof(float), cudaMemcpyDeviceToHost));
-    if (loss) MLP_TRY(cudaMemcpy(loss, mlp->loss, sizeof(float), cudaMemcpyDeviceToHost));
     MLP_TRY(cudaGetLastError());
+    // Through pinned memory: straight into the caller's pageable arrays the
+    // driver stages the copies itself, one after the other.
+    if (host_grads)
+        MLP_TRY(cudaMemcpyAsync(mlp->staged, mlp->g, mlp->nparams * sizeof(float), cudaMemcpyDeviceToHost, s));
+    MLP_TRY(cudaMemcpyAsync(mlp->staged + mlp->nparams, mlp->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
+    MLP_TRY(cudaStreamSynchronize(s));
+    if (host_grads) std::memcpy(host_grads, mlp->staged, mlp->nparams * sizeof(float));
+    if (loss) *loss = mlp->staged[mlp->nparams];
     return BINE_SUCCESS;
 }
 
 int bine_mlp_train_step(bine_mlp_t mlp, const float* d_x, const float* d_t, const float* d_mask, int n, float lr,
                         void* stream, float* loss) {
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = load_batch(mlp, d_x, n, s);
+    int rc = check_targets(d_t, d_mask);
+    if (rc == BINE_SUCCESS) rc = prepare_batch(mlp, d_x, d_mask, n, s);
     if (rc) return rc;
-    forward(mlp, n, s);
-    rc = loss_and_grad(mlp, d_t, d_mask, n, s);
-    if (rc) return rc;
+    forward(mlp, n, nullptr, d_t, d_mask, s);
     backward(mlp, n, s);
     mlp->step++;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -565,8 +774,9 @@ int bine_mlp_train_step(bine_mlp_t mlp, const float* d_x, const float* d_t, cons
     k_adam<<<grid1(mlp->nparams), 256, 0, s>>>(mlp->w, mlp->g, mlp->m, mlp->v, mlp->wb, (long long)mlp->nparams, lr, b1,
                                                b2, 1e-8f, c1, c2);
     if (loss) {
-        MLP_TRY(cudaMemcpyAsync(loss, mlp->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
+        MLP_TRY(cudaMemcpyAsync(mlp->staged + mlp->nparams, mlp->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
         MLP_TRY(cudaStreamSynchronize(s));
+        *loss = mlp->staged[mlp->nparams];
     }
     MLP_TRY(cudaGetLastError());
     return BINE_SUCCESS;
