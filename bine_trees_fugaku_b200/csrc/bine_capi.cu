@@ -104,6 +104,8 @@ struct DevFused {
     DevFlow flow;
     int64_t tmp_elems = 0;
     int npasses = 0;
+    bool copies = true;  // no additions: the kernel's form for copies
+    int resident = 1;    // blocks of that form on the device at once
     ~DevFused() {
         cudaFree(moves);
         cudaFree(leaves);
@@ -113,7 +115,8 @@ struct DevFused {
 static_assert(sizeof(FusedMove) == sizeof(dev::FusedMoveDev), "fused move layouts differ");
 static_assert(sizeof(FusedLeaf) == sizeof(dev::FusedLeafDev), "fused leaf layouts differ");
 static_assert(sizeof(FusedDst) == sizeof(dev::FusedDstDev), "fused destination layouts differ");
-static_assert(dev::kFuseLeaves == kFuseMaxLeaves && dev::kFuseDsts == kFuseMaxDsts, "fusion bounds differ");
+static_assert(dev::kFuseLeaves == kFuseMaxLeaves && dev::kFuseDsts == kFuseMaxDsts && dev::kFuseDepth == kFuseMaxDepth,
+              "fusion bounds differ");
 static_assert((int)BINE_COLL_ALLREDUCE == kAllreduce && (int)BINE_COLL_REDUCE_SCATTER == kReduceScatter &&
                   (int)BINE_COLL_ALLGATHER == kAllgather && (int)BINE_COLL_GATHER == kGather,
               "collective codes differ");
@@ -582,6 +585,9 @@ int fused_schedule(bine_comm_t c, const PlanKey& k, int levels, std::shared_ptr<
 // reductions run fastest at 6 (allreduce B 2.32 TB/s against 2.05 at 10),
 // the copies at 10 and more (allgather 5.07 TB/s against 1.99 at 6);
 // alltoall has about three IR levels per Bine step, and 13 keeps two passes.
+// With sums of up to 16 leaves, 6 stays the best for reductions (allreduce B at
+// P = 256, 1 MiB per rank: 126 us, 148 / 128 / 146 at 5 / 7 / 8; P = 96, 4 MiB:
+// 200, 200 / 337 / 369).
 constexpr int kAutoFusion[kNumColls] = {6, 6, 12, 12, 6, 13, 12, 12};
 
 // Planning a fused schedule costs about 4 us per move on the host (11 s for
@@ -595,6 +601,9 @@ int fusion_levels(bine_comm_t c, int coll, const Schedule* s = nullptr) {
         int64_t moves = 0;
         for (const auto& lvl : s->levels) moves += (int64_t)lvl.size();
         if (moves > kAutoFusionMaxMoves) return 1;
+        // Up to kFuseMaxDsts ranks, every sum and every fan-out fits one move
+        // (allreduce at P = 8, 4 MiB per rank: 26.8 us in two passes, 19.0).
+        if (c->P <= kFuseMaxDsts) return std::max(kAutoFusion[coll], (int)s->levels.size());
     }
     return kAutoFusion[coll];
 }
@@ -602,18 +611,21 @@ int fusion_levels(bine_comm_t c, int coll, const Schedule* s = nullptr) {
 // Blocks of k_flow_fused resident on the device at once: the fused plan
 // cuts each pass into a whole multiple of this many items of equal traffic,
 // so that a pass runs in whole waves.
-int fused_resident_blocks(bine_comm_t c, int es) {
+template <typename T>
+int fused_blocks_per_sm(bool copies) {
     int per_sm = 0;
-    cudaError_t e;
-    switch (es) {
-        case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_flow_fused<int8_t>, dev::kFlowThreads, 0); break;
-        case 8: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_flow_fused<int64_t>, dev::kFlowThreads, 0); break;
-        default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_flow_fused<int32_t>, dev::kFlowThreads, 0);
-    }
-    if (e != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        per_sm = kFlowItemsPerSm;
-    }
+    const cudaError_t e =
+        copies ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_flow_fused<T, 1>, dev::kFlowThreads, 0)
+               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_flow_fused<T, dev::kFuseLeaves>,
+                                                               dev::kFlowThreads, 0);
+    if (e == cudaSuccess && per_sm >= 1) return per_sm;
+    cudaGetLastError();
+    return kFlowItemsPerSm;
+}
+
+int fused_resident_blocks(bine_comm_t c, int es, bool copies) {
+    const int per_sm = es == 1 ? fused_blocks_per_sm<int8_t>(copies)
+                               : (es == 8 ? fused_blocks_per_sm<int64_t>(copies) : fused_blocks_per_sm<int32_t>(copies));
     return per_sm * c->num_sms;
 }
 
@@ -645,7 +657,7 @@ int get_dev_fused(bine_comm_t c, const PlanKey& k, int es, std::shared_ptr<DevFu
             for (int j = 0; j < m.nleaves; j++) {
                 const FusedLeaf& lf = fs.leaves[m.leaf_begin + j];
                 if (lf.rank < 0 || lf.rank >= c->P || lf.buf > kBufTmp || lf.off < 0 || lf.off + m.n > rows[lf.buf] ||
-                    (j == 0 && lf.adds != 0) || lf.adds > 3)
+                    (j == 0 && lf.adds != 0) || lf.adds >= kFuseMaxDepth)
                     return fail(BINE_ERR_INTERNAL, "fusion produced a leaf outside its buffer row");
                 maxd = std::max(maxd, depth + 1);  // the leaf is pushed before its additions
                 depth += 1 - lf.adds;
@@ -659,14 +671,17 @@ int get_dev_fused(bine_comm_t c, const PlanKey& k, int es, std::shared_ptr<DevFu
                     return fail(BINE_ERR_INTERNAL, "fusion produced a destination outside its buffer row");
             }
         }
+    auto d = std::make_shared<DevFused>();
+    for (const auto& pass : fs.passes)
+        for (const FusedMove& m : pass) d->copies = d->copies && m.nleaves == 1;
+    d->resident = fused_resident_blocks(c, es, d->copies);
     FlowPlan fp;
     // Pieces of at most kFlowMaxItemBytes keep every item below 2^31 bytes,
     // the kernel's 32-bit unit counts.
     const int64_t piece =
         c->segment_bytes > 0 ? std::max<int64_t>(16, std::min<int64_t>(c->segment_bytes, kFlowMaxItemBytes) / es) : 0;
     build_flow_fused(fs, c->P, piece, std::max<int64_t>(1, 4096 / es), kFlowMaxItemBytes / es,
-                     fused_resident_blocks(c, es), dev::kFusedPieces, &fp);
-    auto d = std::make_shared<DevFused>();
+                     d->resident, dev::kFusedPieces, &fp);
     d->tmp_elems = fs.tmp_elems;
     d->npasses = (int)fs.passes.size();
     std::vector<FusedMove> moves;
@@ -1780,7 +1795,7 @@ int launch_flow(bine_comm_t c, const DevSteps& d, const DevFlow& f, const char* 
     return BINE_SUCCESS;
 }
 
-template <typename T>
+template <typename T, int L>
 int launch_flow_fused(bine_comm_t c, const DevFused& d, const char* send, long long ist, char* recv, long long ost) {
     const DevFlow& f = d.flow;
     if (f.nitems == 0) return BINE_SUCCESS;
@@ -1795,10 +1810,8 @@ int launch_flow_fused(bine_comm_t c, const DevFused& d, const char* send, long l
     B.stride[kBufSend] = ist;
     B.stride[kBufRecv] = ost;
     B.stride[kBufTmp] = (long long)tmp_stride;
-    int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_flow_fused<T>, dev::kFlowThreads, 0));
-    const int blocks = std::max(1, std::min(std::max(1, per_sm) * c->num_sms, f.nitems));
-    dev::k_flow_fused<T><<<blocks, dev::kFlowThreads, 0, c->stream>>>(
+    const int blocks = std::max(1, std::min(d.resident, f.nitems));
+    dev::k_flow_fused<T, L><<<blocks, dev::kFlowThreads, 0, c->stream>>>(
         B, d.moves, d.leaves, d.dsts, f.pieces, f.items, f.nitems, f.deps, f.level_items, f.nlevels, f.done, f.ctl,
         c->status, c->step_timeout_ns, c->barrier_extra);
     CUDA_TRY(cudaGetLastError());
@@ -1807,12 +1820,23 @@ int launch_flow_fused(bine_comm_t c, const DevFused& d, const char* send, long l
 
 int launch_flow_fused_dt(bine_comm_t c, int dt, const DevFused& d, const char* send, long long ist, char* recv,
                          long long ost) {
+    constexpr int L = dev::kFuseLeaves;
     switch (dt) {
-    case BINE_INT32: return launch_flow_fused<int32_t>(c, d, send, ist, recv, ost);
-    case BINE_INT64: return launch_flow_fused<int64_t>(c, d, send, ist, recv, ost);
-    case BINE_FLOAT: return launch_flow_fused<float>(c, d, send, ist, recv, ost);
-    case BINE_DOUBLE: return launch_flow_fused<double>(c, d, send, ist, recv, ost);
-    case BINE_CHAR: return launch_flow_fused<int8_t>(c, d, send, ist, recv, ost);
+    case BINE_INT32:
+        return d.copies ? launch_flow_fused<int32_t, 1>(c, d, send, ist, recv, ost)
+                        : launch_flow_fused<int32_t, L>(c, d, send, ist, recv, ost);
+    case BINE_INT64:
+        return d.copies ? launch_flow_fused<int64_t, 1>(c, d, send, ist, recv, ost)
+                        : launch_flow_fused<int64_t, L>(c, d, send, ist, recv, ost);
+    case BINE_FLOAT:  // copies: by element size
+        return d.copies ? launch_flow_fused<int32_t, 1>(c, d, send, ist, recv, ost)
+                        : launch_flow_fused<float, L>(c, d, send, ist, recv, ost);
+    case BINE_DOUBLE:
+        return d.copies ? launch_flow_fused<int64_t, 1>(c, d, send, ist, recv, ost)
+                        : launch_flow_fused<double, L>(c, d, send, ist, recv, ost);
+    case BINE_CHAR:
+        return d.copies ? launch_flow_fused<int8_t, 1>(c, d, send, ist, recv, ost)
+                        : launch_flow_fused<int8_t, L>(c, d, send, ist, recv, ost);
     }
     return fail(BINE_ERR_ARG, "bad datatype");
 }

@@ -9,8 +9,8 @@
 // inside the pass, staged messages, copies overwritten before use) is never
 // written.  The kept runs become fused moves: a postfix program over leaves
 // (at most kFuseMaxLeaves, stack depth at most kFuseMaxDepth) and the rows
-// it is written to.  Passes whose kept writes overlap what another of their
-// moves reads, or whose programs are too large, are split until none is.
+// it is written to.  A pass ends early, before the level whose programs would
+// be too large.
 // Finally the fused schedule is executed symbolically from the collective's
 // inputs beside the original one, in one hash-consed expression table, and
 // every result element must come out as the same addition tree.
@@ -66,6 +66,12 @@ class Exec {
         return id;
     }
     const FNode& node(int32_t id) const { return nodes_[id]; }
+    // Whether every value computed so far is within the fused kernel's bounds.
+    bool within_bounds() {
+        for (; checked_ < nodes_.size() && fits_; checked_++)
+            fits_ = nodes_[checked_].leaves <= kFuseMaxLeaves && nodes_[checked_].depth <= kFuseMaxDepth;
+        return fits_;
+    }
     void clear_state() { rows_.clear(); }
     const std::unordered_map<uint64_t, Runs>& rows() const { return rows_; }
 
@@ -202,6 +208,8 @@ class Exec {
         }
     }
     std::vector<FNode> nodes_;
+    size_t checked_ = 0;  // nodes that within_bounds has looked at
+    bool fits_ = true;
     std::map<std::tuple<int32_t, int32_t, int64_t>, int32_t> memo_;
     std::unordered_map<uint64_t, int32_t> leaf_ids_;
     std::unordered_map<uint64_t, Runs> rows_;
@@ -270,11 +278,20 @@ struct PassSym {
     std::vector<Write> writes;  // every run the pass changes, sorted by row and offset
 };
 
-PassSym run_pass(const Schedule& sch, int a, int b) {
+// Executes levels [a, b); with `end`, stops before the first level after a
+// whose values are too large for the kernel and returns where it stopped.
+PassSym run_pass(const Schedule& sch, int a, int b, int* end = nullptr) {
     PassSym ps;
     ps.ex.reset(new Exec());
     Exec& ex = *ps.ex;
-    for (int l = a; l < b; l++) ex.apply_level(sch.levels[l]);
+    for (int l = a; l < b; l++) {
+        ex.apply_level(sch.levels[l]);
+        if (end && !ex.within_bounds() && l > a) {
+            *end = l;
+            return run_pass(sch, a, l);
+        }
+    }
+    if (end) *end = b;
     for (const auto& kv : ex.rows()) {
         const int rank = (int)(kv.first >> 8), buf = (int)(kv.first & 0xFF);
         const FVal id{ex.leaf(rank, buf), 0};
@@ -469,68 +486,55 @@ bool fuse_schedule(const Schedule& sch, int P, int depth, const std::vector<bool
     *out = FusedSchedule();
     const int L = (int)sch.levels.size();
     depth = std::max(1, depth);
-    std::vector<int> bounds;  // pass starts, then L
-    for (int l = 0; l < L; l += depth) bounds.push_back(l);
-    bounds.push_back(L);
-    std::map<std::pair<int, int>, PassSym> cache;
-    std::vector<std::vector<Write>> kept;
-    std::vector<PassSym*> ps;
-    for (int iter = 0;; iter++) {
-        if (iter > 4 * L + 8) {
-            *err = "fusion: splitting passes did not converge";
-            return false;
+    // A pass ends before the level whose sums outgrow
+    // the kernel's programs, and the next one starts there: early passes as
+    // long as they can be, since the partial sums that a pass writes halve
+    // with each of its levels.  Allreduce B at P = 256 moves 1.13 times the
+    // algorithmic bytes in 3 passes of 5, 6 and 6 levels; passes of 6 levels
+    // halved where they were too large moved 1.34 times in 4 (of 3, 3, 6, 5).  What follows is
+    // cut evenly into as few passes as `depth` allows: at P = 64, 5, 4 and 4
+    // levels and no results left in slots (4 MiB per rank 126 us, with 5, 6
+    // and 2 levels 144).
+    std::vector<PassSym> ps;
+    std::vector<int> pass_levels;
+    for (int l = 0, step = depth; l < L;) {
+        const int goal = std::min(L, l + step);
+        int end = goal;
+        ps.push_back(run_pass(sch, l, goal, &end));
+        pass_levels.push_back(end - l);
+        l = end;
+        const int rest = (L - l + depth - 1) / depth;  // passes
+        if (end < goal && rest > 0) step = (L - l + rest - 1) / rest;
+    }
+    const int np = (int)ps.size();
+    // Backward liveness: a run is kept when a later pass reads it or it
+    // is a result; what a kept run reads is live before its pass.
+    std::unordered_map<uint64_t, ISet> live;
+    for (int r = 0; r < P; r++)
+        if (out_rows[r] && sch.recv_elems > 0) iset_add(live[row_key(r, kBufRecv)], 0, sch.recv_elems);
+    std::vector<std::vector<Write>> kept(np);
+    std::vector<std::tuple<int32_t, uint8_t, int64_t>> lv;
+    for (int p = np - 1; p >= 0; p--) {
+        for (const Write& w : ps[p].writes) {
+            auto lit = live.find(row_key(w.rank, w.buf));
+            if (lit == live.end()) continue;
+            for (auto& iv : iset_meet(lit->second, w.s, w.e))
+                kept[p].push_back(Write{w.rank, w.buf, iv.first, iv.second, w.v});
         }
-        const int np = (int)bounds.size() - 1;
-        ps.assign(np, nullptr);
-        for (int p = 0; p < np; p++) {
-            const auto key = std::make_pair(bounds[p], bounds[p + 1]);
-            auto it = cache.find(key);
-            if (it == cache.end()) it = cache.emplace(key, run_pass(sch, key.first, key.second)).first;
-            ps[p] = &it->second;
+        for (const Write& w : ps[p].writes) {
+            auto lit = live.find(row_key(w.rank, w.buf));
+            if (lit != live.end()) iset_sub(lit->second, w.s, w.e);
         }
-        // Backward liveness: a run is kept when a later pass reads it or it
-        // is a result; what a kept run reads is live before its pass.
-        std::unordered_map<uint64_t, ISet> live;
-        for (int r = 0; r < P; r++)
-            if (out_rows[r] && sch.recv_elems > 0) iset_add(live[row_key(r, kBufRecv)], 0, sch.recv_elems);
-        kept.assign(np, {});
-        std::vector<std::tuple<int32_t, uint8_t, int64_t>> lv;
-        for (int p = np - 1; p >= 0; p--) {
-            for (const Write& w : ps[p]->writes) {
-                auto lit = live.find(row_key(w.rank, w.buf));
-                if (lit == live.end()) continue;
-                for (auto& iv : iset_meet(lit->second, w.s, w.e))
-                    kept[p].push_back(Write{w.rank, w.buf, iv.first, iv.second, w.v});
+        for (const Write& k : kept[p]) {
+            const FNode& n = ps[p].ex->node(k.v.node);
+            if (n.leaves > kFuseMaxLeaves || n.depth > kFuseMaxDepth) {
+                *err = "fusion: a level has a program too large";
+                return false;
             }
-            for (const Write& w : ps[p]->writes) {
-                auto lit = live.find(row_key(w.rank, w.buf));
-                if (lit != live.end()) iset_sub(lit->second, w.s, w.e);
-            }
-            for (const Write& k : kept[p]) {
-                lv.clear();
-                ps[p]->ex->leaves_of(k.v.node, k.v.shift, &lv);
-                for (auto& t : lv)
-                    iset_add(live[row_key(std::get<0>(t), std::get<1>(t))], k.s + std::get<2>(t), k.e + std::get<2>(t));
-            }
-        }
-        // A pass whose programs are too large for the kernel is split.
-        std::vector<int> bad;
-        for (int p = 0; p < np; p++)
-            for (const Write& k : kept[p]) {
-                const FNode& n = ps[p]->ex->node(k.v.node);
-                if (n.leaves > kFuseMaxLeaves || n.depth > kFuseMaxDepth) {
-                    if (bounds[p + 1] - bounds[p] == 1) {
-                        *err = "fusion: level " + std::to_string(bounds[p]) + " has a program too large";
-                        return false;
-                    }
-                    bad.push_back(p);
-                    break;
-                }
-            }
-        if (bad.empty()) break;
-        for (int j = (int)bad.size() - 1; j >= 0; j--) {
-            const int p = bad[j];
-            bounds.insert(bounds.begin() + p + 1, (bounds[p] + bounds[p + 1]) / 2);
+            lv.clear();
+            ps[p].ex->leaves_of(k.v.node, k.v.shift, &lv);
+            for (auto& t : lv)
+                iset_add(live[row_key(std::get<0>(t), std::get<1>(t))], k.s + std::get<2>(t), k.e + std::get<2>(t));
         }
     }
     // Forward: place every pass's writes and emit its moves, one per group
@@ -539,7 +543,6 @@ bool fuse_schedule(const Schedule& sch, int P, int depth, const std::vector<bool
     std::vector<int64_t> cursor(P, 0);
     const int64_t slot_base = sch.tmp_elems;
     std::vector<Sub> subs;
-    const int np = (int)bounds.size() - 1;
     auto emit_pass = [&](const std::vector<Sub>& sb, int levels) {
         std::map<int32_t, std::vector<const Sub*>> groups;
         for (const Sub& x : sb) groups[x.group].push_back(&x);
@@ -569,8 +572,8 @@ bool fuse_schedule(const Schedule& sch, int P, int depth, const std::vector<bool
         }
     };
     for (int p = 0; p < np; p++) {
-        place_pass(*ps[p]->ex, kept[p], pl, slot_base, cursor, &subs);
-        emit_pass(subs, bounds[p + 1] - bounds[p]);
+        place_pass(*ps[p].ex, kept[p], pl, slot_base, cursor, &subs);
+        emit_pass(subs, pass_levels[p]);
     }
     // Results still in renaming slots are copied home.
     subs.clear();

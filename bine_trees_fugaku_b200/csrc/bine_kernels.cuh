@@ -1608,16 +1608,26 @@ __global__ void __launch_bounds__(kFlowThreads, kFlowBlocksPerSm) k_flow(StepBuf
 // bine_plan.h): a piece belongs to a fused move whose value is a postfix
 // program over at most kFuseLeaves state elements, written to at most
 // kFuseDsts destinations.  Each unit (a 16-byte vector, or an element at a
-// piece's unaligned head and tail) loads all of its leaves, evaluates the
-// program on a four-entry stack (the top in registers, the rest in shared
-// memory for 16-byte units) in the order of the original levels'
-// additions, and stores the value to every destination; the loads
-// come before the stores, so a move may update its own elements in place.
-// Items of copies only (one leaf per program: the gather and alltoall
-// passes) move four 16-byte units per thread and round, other items one
-// unit with all its leaves in flight.  Three blocks of 256 threads per SM
-// (80 registers): the planner cuts each pass into a whole multiple of the
-// resident blocks' count of equal-traffic items.
+// piece's unaligned head and tail) loads its leaves eight at a time,
+// evaluates the program in the order of the original levels' additions (full
+// binary trees in registers, others on a five-entry stack in shared memory),
+// and stores the value to every destination; all loads come before the
+// stores, so a move may update its own elements in place.  Items of copies
+// only (the gather and alltoall passes) move four 16-byte units per thread
+// and round, other items one unit with eight leaves in flight.  The planner
+// cuts each pass into a whole multiple of the resident blocks' count of
+// equal-traffic items.
+//
+// Bound by DRAM and L2 traffic for large rows, by the chain of dependent loads
+// per item (three table rounds, the wait, the data) for small ones.  Programs
+// of up to 16 leaves instead of 8 take allreduce B at P = 256 from 1.34 to
+// 1.13 times the algorithmic bytes and from four passes to three; us per call
+// on B200, float32, 8 leaves -> 16: 1 MiB per rank 165 -> 129, 4 MiB 564 ->
+// 442, 400,004 bytes 154 -> 105; P = 96, 4 MiB 305 -> 202; P = 64, 8 KiB 20.5
+// -> 16.9; reduce_scatter at P = 128, 1 MiB 62 -> 44.  Schedules of copies
+// have a form of their own (FusedItemSmem<1>: 14 of 47 KiB, 64 registers,
+// four blocks per SM instead of three of 80): alltoall at P = 128, 1 MiB 128
+// -> 107 us; in the 16-leaf form it took 142.
 struct FusedMoveDev {
     int64_t n;
     int32_t leaf_begin, nleaves, dst_begin, ndst;
@@ -1632,53 +1642,30 @@ struct FusedDstDev {
     uint8_t buf, pad[3];
     int64_t off;
 };
-constexpr int kFuseLeaves = 8;
+constexpr int kFuseLeaves = 16;
 constexpr int kFuseDsts = 8;
+constexpr int kFuseDepth = 5;      // evaluation stack, the top included
+constexpr int kFuseRound = 8;      // leaves of a 16-byte unit loaded at once
 constexpr int kFusedPieces = 128;  // pieces per item, at most one per thread
 static_assert(kFusedPieces <= kFlowThreads, "one thread per piece of an item");
-
-// Postfix evaluation of at most L leaves on a shift-register stack (s0 is
-// the top): a leaf pushes, each addition pops the top two and pushes their
-// sum.  IEEE and wrapping integer addition are commutative, so only the
-// tree's shape matters, and it is the program's.
-template <int L, typename V, typename Add>
-__device__ __forceinline__ V fused_eval(const V* v, const unsigned char* adds, int nl, Add add) {
-    V s0 = v[0], s1 = v[0], s2 = v[0], s3 = v[0];
-#pragma unroll
-    for (int j = 1; j < L; j++) {
-        if (j < nl) {
-            s3 = s2;
-            s2 = s1;
-            s1 = s0;
-            s0 = v[j];
-            const int na = adds[j];
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-                if (a < na) {
-                    s0 = add(s1, s0);
-                    s1 = s2;
-                    s2 = s3;
-                }
-        }
-    }
-    return s0;
-}
 
 // Per-item tables of k_flow_fused: every piece's leaf and destination
 // addresses, its evaluation program, and block scans of its 16-byte units
 // and of its element units (an unaligned head and tail, or the whole piece
 // when its rows are not mutually 16-byte aligned).  The planner keeps an
 // item below 2^31 elements, so unit counts fit 32 bits.
+template <int L>
 struct FusedItemSmem {
     int pref[kFusedPieces + 1];   // first 16-byte unit of each piece
     int epref[kFusedPieces + 1];  // first element unit of each piece
-    const char* leaf[kFusedPieces][kFuseLeaves];
+    const char* leaf[kFusedPieces][L];
     char* dst[kFusedPieces][kFuseDsts];
     long long start[kFusedPieces], n[kFusedPieces];
     int nvec[kFusedPieces], lb[kFusedPieces], db[kFusedPieces];
-    unsigned char adds[kFusedPieces][kFuseLeaves];
+    unsigned char adds[kFusedPieces][L];
     unsigned char head[kFusedPieces], nl[kFusedPieces], nd[kFusedPieces];
-    uint4 stk[3][kFlowThreads];  // evaluation stack below the top (depth <= 4), per thread
+    unsigned char full[kFusedPieces];  // the program is a full binary tree
+    uint4 stk[L > 1 ? kFuseDepth - 1 : 1][L > 1 ? kFlowThreads : 1];  // evaluation stack below the top, per thread
     char* base[3];               // the launch's buffer rows (StepBufs), read from shared memory
     long long stride[3];
     long long warp_sum[kFlowThreads / 32];
@@ -1698,18 +1685,16 @@ __device__ __forceinline__ int fused_piece(const int* pref, int u, int np, int c
     return lo;
 }
 
-// The 16-byte units of an item whose programs have at most L leaves (L = 1:
-// copies; L = 2: single additions): U units per thread and round, every
-// unit's loads issued before the round's stores.  Units of one item touch
+// The 16-byte units of an item of copies: U units per thread and round, every
+// unit's load issued before the round's stores.  Units of one item touch
 // disjoint elements apart from a move's in-place reads of its own elements,
 // so the order of rounds and units does not matter.
 template <typename T, int U, int L>
-__device__ __forceinline__ void fused_units_narrow(const FusedItemSmem& S, int tid, int total, int np) {
-    static_assert(L == 1 || L == 2, "narrow programs only");
+__device__ __forceinline__ void fused_units_copy(const FusedItemSmem<L>& S, int tid, int total, int np) {
     constexpr int es = sizeof(T);
     int cur = 0;
     for (int u0 = tid; u0 < total; u0 += U * kFlowThreads) {
-        uint4 v[U][L];
+        uint4 v[U];
         int pc[U], off[U];
 #pragma unroll
         for (int k = 0; k < U; k++) {
@@ -1720,78 +1705,108 @@ __device__ __forceinline__ void fused_units_narrow(const FusedItemSmem& S, int t
                 cur = fused_piece(S.pref, u, np, cur);
                 pc[k] = cur;
                 off[k] = S.head[cur] * es + (u - S.pref[cur]) * 16;
-                v[k][0] = ld_plain(S.leaf[cur][0] + off[k]);
-                if (L == 2 && S.nl[cur] == 2) v[k][L - 1] = ld_plain(S.leaf[cur][L - 1] + off[k]);
+                v[k] = ld_plain(S.leaf[cur][0] + off[k]);
             }
         }
 #pragma unroll
         for (int k = 0; k < U; k++) {
             if (pc[k] < 0) continue;
             const int p = pc[k];
-            const uint4 val = (L == 2 && S.nl[p] == 2) ? vadd<T>(v[k][0], v[k][L - 1]) : v[k][0];
             const int nd = S.nd[p];
 #pragma unroll
             for (int j = 0; j < kFuseDsts; j++)
-                if (j < nd) *(uint4*)(S.dst[p][j] + off[k]) = val;
+                if (j < nd) *(uint4*)(S.dst[p][j] + off[k]) = v[k];
         }
     }
 }
 
-// The 16-byte units of any item: one unit per thread and round, its leaves
-// loaded together, the program evaluated with the entries below the top of
-// its stack in this thread's column of S.stk (registers would cost the
-// third block per SM).
-template <typename T>
-__device__ __forceinline__ void fused_units_wide(FusedItemSmem& S, int tid, int total, int np) {
+// The value of one unit of piece p (V: a 16-byte vector, or one element),
+// leaves loaded eight at a time by ld(leaf).  Full binary trees (the sums of
+// the halving and butterfly steps) are added in registers; other programs
+// keep the entries below the top of their stack in this thread's column of
+// S.stk (registers would cost the third block per SM).  IEEE and wrapping
+// integer addition are commutative, so only the tree's shape matters, and it
+// is the program's.
+template <typename V, int L, typename Ld, typename Add>
+__device__ __forceinline__ V fused_value(FusedItemSmem<L>& S, int tid, int p, Ld ld, Add add) {
+    static_assert(kFuseRound == 8 && L == 16, "two rounds of eight leaves");
+    const int nl = S.nl[p];
+    V v[kFuseRound];
+    if (S.full[p]) {  // 1, 2, 4, 8 or 16 leaves
+#pragma unroll
+        for (int j = 0; j < kFuseRound; j++)
+            if (j < nl) v[j] = ld(S.leaf[p][j]);
+        V top = v[0];
+        if (nl > 1) top = add(top, v[1]);
+        if (nl > 2) top = add(top, add(v[2], v[3]));
+        if (nl > 4) top = add(top, add(add(v[4], v[5]), add(v[6], v[7])));
+        if (nl > 8) {
+#pragma unroll
+            for (int j = 0; j < kFuseRound; j++) v[j] = ld(S.leaf[p][kFuseRound + j]);
+            top = add(top, add(add(add(v[0], v[1]), add(v[2], v[3])), add(add(v[4], v[5]), add(v[6], v[7]))));
+        }
+        return top;
+    }
+    V top;
+    int sp = 0;
+#pragma unroll 1
+    for (int r = 0; r < nl; r += kFuseRound) {
+#pragma unroll
+        for (int j = 0; j < kFuseRound; j++)
+            if (r + j < nl) v[j] = ld(S.leaf[p][r + j]);
+#pragma unroll
+        for (int j = 0; j < kFuseRound; j++)
+            if (r + j < nl) {
+                if (r + j > 0) *(V*)&S.stk[sp++][tid] = top;
+                top = v[j];
+                for (int a = S.adds[p][r + j]; a > 0; a--) top = add(*(const V*)&S.stk[--sp][tid], top);
+            }
+    }
+    return top;
+}
+
+// The 16-byte units of any item, one per thread and round.
+template <typename T, int L>
+__device__ __forceinline__ void fused_units_wide(FusedItemSmem<L>& S, int tid, int total, int np) {
     constexpr int es = sizeof(T);
     int cur = 0;
     for (int u = tid; u < total; u += kFlowThreads) {
         cur = fused_piece(S.pref, u, np, cur);
-        const int off = S.head[cur] * es + (u - S.pref[cur]) * 16;
-        const int nl = S.nl[cur], nd = S.nd[cur];
-        uint4 v[kFuseLeaves];
-#pragma unroll
-        for (int j = 0; j < kFuseLeaves; j++)
-            if (j < nl) v[j] = ld_plain(S.leaf[cur][j] + off);
-        uint4 top = v[0];
-        int sp = 0;
-#pragma unroll
-        for (int j = 1; j < kFuseLeaves; j++)
-            if (j < nl) {
-                S.stk[sp++][tid] = top;
-                top = v[j];
-                for (int a = S.adds[cur][j]; a > 0; a--) top = vadd<T>(S.stk[--sp][tid], top);
-            }
+        const int off = S.head[cur] * es + (u - S.pref[cur]) * 16, nd = S.nd[cur];
+        const uint4 val = fused_value<uint4>(S, tid, cur, [&](const char* p) { return ld_plain(p + off); },
+                                             [](uint4 x, uint4 y) { return vadd<T>(x, y); });
 #pragma unroll
         for (int j = 0; j < kFuseDsts; j++)
-            if (j < nd) *(uint4*)(S.dst[cur][j] + off) = top;
+            if (j < nd) *(uint4*)(S.dst[cur][j] + off) = val;
     }
 }
 
 // The element units of an item: a piece's unaligned head, its tail after
 // the 16-byte body, or all of a piece without one.
-template <typename T>
-__device__ __forceinline__ void fused_elements(const FusedItemSmem& S, int tid, int total, int np) {
+template <typename T, int L>
+__device__ __forceinline__ void fused_elements(FusedItemSmem<L>& S, int tid, int total, int np) {
     constexpr int per_vec = 16 / sizeof(T);
     int cur = 0;
     for (int u = tid; u < total; u += kFlowThreads) {
         cur = fused_piece(S.epref, u, np, cur);
         const long long r = u - S.epref[cur];
         const long long e = r < S.head[cur] ? r : r + (long long)S.nvec[cur] * per_vec;
-        const int nl = S.nl[cur], nd = S.nd[cur];
-        T w[kFuseLeaves];
-#pragma unroll
-        for (int j = 0; j < kFuseLeaves; j++)
-            if (j < nl) w[j] = *((volatile const T*)S.leaf[cur][j] + e);
-        const T val = fused_eval<kFuseLeaves>(w, S.adds[cur], nl, [](T x, T y) { return add_exact<T>(x, y); });
+        const int nd = S.nd[cur];
+        T val;
+        if constexpr (L == 1)
+            val = *((volatile const T*)S.leaf[cur][0] + e);
+        else
+            val = fused_value<T>(S, tid, cur, [&](const char* p) { return *((volatile const T*)p + e); },
+                                 [](T x, T y) { return add_exact<T>(x, y); });
 #pragma unroll
         for (int j = 0; j < kFuseDsts; j++)
             if (j < nd) *((T*)S.dst[cur][j] + e) = val;
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kFlowThreads, 3) k_flow_fused(StepBufs B, const FusedMoveDev* __restrict__ moves,
+// L: the longest program of the schedule, 1 (copies only) or kFuseLeaves.
+template <typename T, int L>
+__global__ void __launch_bounds__(kFlowThreads, L == 1 ? 4 : 3) k_flow_fused(StepBufs B, const FusedMoveDev* __restrict__ moves,
                                                             const FusedLeafDev* __restrict__ leaves,
                                                             const FusedDstDev* __restrict__ dsts,
                                                             const StepChunk* __restrict__ pieces,
@@ -1800,7 +1815,8 @@ __global__ void __launch_bounds__(kFlowThreads, 3) k_flow_fused(StepBufs B, cons
                                                             const int* __restrict__ level_items, int nlevels,
                                                             unsigned* done, unsigned* ctl, int* status,
                                                             unsigned long long timeout_ns, unsigned extra) {
-    __shared__ FusedItemSmem S;
+    __shared__ FusedItemSmem<L> S;
+    static_assert(sizeof(FusedItemSmem<L>) <= 48 * 1024, "static shared memory");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         const unsigned t = ld_acquire(&ctl[2]) + 1u;
@@ -1813,7 +1829,7 @@ __global__ void __launch_bounds__(kFlowThreads, 3) k_flow_fused(StepBufs B, cons
     __syncthreads();
     const unsigned target = S.target;
     constexpr long long es = sizeof(T);
-    constexpr int kSlots = kFuseLeaves + kFuseDsts;
+    constexpr int kSlots = L + kFuseDsts;
     for (;;) {
         if (tid == 0) {
             S.item = *(volatile int*)status == kStepOk ? (int)atomicAdd(&ctl[0], 1u) : nitems;
@@ -1842,16 +1858,16 @@ __global__ void __launch_bounds__(kFlowThreads, 3) k_flow_fused(StepBufs B, cons
 #pragma unroll 4
         for (int e = tid; e < np * kSlots; e += kFlowThreads) {
             const int p = e / kSlots, j = e % kSlots;
-            if (j < kFuseLeaves) {
+            if (j < L) {
                 if (j < S.nl[p]) {
                     const FusedLeafDev lf = leaves[S.lb[p] + j];
                     S.leaf[p][j] =
                         S.base[lf.buf] + (long long)lf.rank * S.stride[lf.buf] + (lf.off + S.start[p]) * es;
                     S.adds[p][j] = lf.adds;
                 }
-            } else if (j - kFuseLeaves < S.nd[p]) {
-                const FusedDstDev d = dsts[S.db[p] + j - kFuseLeaves];
-                S.dst[p][j - kFuseLeaves] =
+            } else if (j - L < S.nd[p]) {
+                const FusedDstDev d = dsts[S.db[p] + j - L];
+                S.dst[p][j - L] =
                     S.base[d.buf] + (long long)d.rank * S.stride[d.buf] + (d.off + S.start[p]) * es;
             }
         }
@@ -1872,6 +1888,10 @@ __global__ void __launch_bounds__(kFlowThreads, 3) k_flow_fused(StepBufs B, cons
             units = ((n - nvec * (16 / es)) << 32) | nvec;
             S.nvec[tid] = (int)nvec;
             S.head[tid] = (unsigned char)head;
+            const int nl = S.nl[tid];
+            bool full = (nl & (nl - 1)) == 0;
+            for (int j = 1; j < nl; j++) full = full && S.adds[tid][j] == __ffs(j + 1) - 1;
+            S.full[tid] = full;
         }
         long long inc = units;
 #pragma unroll
@@ -1898,10 +1918,9 @@ __global__ void __launch_bounds__(kFlowThreads, 3) k_flow_fused(StepBufs B, cons
         __syncthreads();
         if (!S.ok) break;  // a wait expired; the status is recorded
         const int total = S.pref[np];
-        const int maxnl = S.maxnl;
-        if (maxnl <= 1)
-            fused_units_narrow<T, 4, 1>(S, tid, total, np);
-        else
+        if (L == 1 || S.maxnl <= 1)
+            fused_units_copy<T, 4>(S, tid, total, np);
+        else if constexpr (L > 1)
             fused_units_wide<T>(S, tid, total, np);
         if (S.epref[np] > 0) fused_elements<T>(S, tid, S.epref[np], np);
         __syncthreads();

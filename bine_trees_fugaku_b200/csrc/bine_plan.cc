@@ -2026,8 +2026,12 @@ void pack_balanced(const std::vector<int64_t>& sizes, const std::vector<int32_t>
     // goal * (max_pieces - 1) >= moves keeps items within max_pieces.
     const int64_t tp = (int64_t)target_items * std::max(1, max_pieces - 1);
     const int64_t waves = std::max<int64_t>({1, (level_w + tw - 1) / tw, ((int64_t)sizes.size() + tp - 1) / tp});
-    // Levels too small for that get items of 2 * min_item_elems accesses.
-    const int64_t goal = std::max<int64_t>(1, std::min(waves * target_items, level_w / (2 * min_item_elems)));
+    // Levels too small for that get items of 2 * min_item_elems accesses, or
+    // of 32 moves where that is less: an item's tables cost more than its data
+    // when it has many short moves (allreduce at P = 256, us: 512 bytes per
+    // rank 29.2 without / 24.2 with 32 / 28.2 with 16; 8 KiB 25.3 / 24.0 / 29.1).
+    const int64_t small = std::max<int64_t>(level_w / (2 * min_item_elems), (int64_t)sizes.size() / 32);
+    const int64_t goal = std::max<int64_t>(1, std::min(waves * target_items, small));
     // Item k ends where the level's accesses reach (k + 1) / goal of the
     // total; a move is cut at the multiple of min_item_elems nearest that
     // boundary.  An item that reaches max_pieces first is continued by a

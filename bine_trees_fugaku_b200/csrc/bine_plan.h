@@ -239,15 +239,15 @@ struct FusedSchedule {
     std::vector<int32_t> pass_levels;  // original levels per pass (0: the final copy of renamed results)
     int64_t tmp_elems = 0;             // workspace elements per rank, renaming slots included
 };
-constexpr int kFuseMaxLeaves = 8;  // leaves of one fused value (2^3: three levels of sums)
-constexpr int kFuseMaxDsts = 8;    // destinations of one fused move
-constexpr int kFuseMaxDepth = 4;   // evaluation stack of one program
+constexpr int kFuseMaxLeaves = 16;  // leaves of one fused value (2^4: four levels of sums)
+constexpr int kFuseMaxDsts = 8;     // destinations of one fused move
+constexpr int kFuseMaxDepth = 5;    // evaluation stack of one program
 
 // Fuses up to `depth` consecutive levels per pass (depth 1 keeps every
 // level but still drops writes nothing reads).  `out_rows[r]` tells whether
 // rank r's receive row is a result.  A pass whose values would need more
-// than kFuseMaxLeaves leaves or kFuseMaxDepth stack entries is split.  A
-// write that would overwrite an element another move of its pass still
+// than kFuseMaxLeaves leaves or kFuseMaxDepth stack entries ends before the
+// level that needs them, and the next pass starts there.  A write that would overwrite an element another move of its pass still
 // reads goes to a fresh workspace slot (after the schedule's own workspace)
 // and later passes read it there; results left in slots are copied home by
 // a last pass.  The fused schedule is checked against the original by
