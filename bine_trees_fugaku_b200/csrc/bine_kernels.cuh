@@ -16,8 +16,8 @@
 //                output segment carries the postfix program of its addition
 //                tree (produced by the host planner), evaluated per column
 //                with an in-register top of stack.
-//   k_copy_*     allgather, bcast, alltoall, scatter and gather as one pass of
-//                16-byte copies (one load, one or P stores).
+//   k_copy_*,    allgather, bcast, alltoall, scatter and gather as one pass of
+//   k_spread     16-byte copies (one load, one or P stores).
 //   k_steps      the reference's schedule executed level by level in one
 //                cooperative launch, with a bounded grid-wide barrier between
 //                levels that reports a timeout instead of hanging.
