@@ -547,6 +547,7 @@ struct bine_mlp_s {
     float* losses = nullptr;     // loss per output tile, then the loss
     float* loss = nullptr;
     float* staged = nullptr;     // pinned host copy of the gradients and the loss
+    cudaEvent_t inputs_read = nullptr;  // a step's last read of the caller's arrays
     ~bine_mlp_s() {
         cudaFree(w);
         cudaFree(g);
@@ -560,6 +561,7 @@ struct bine_mlp_s {
         cudaFree(counts);
         cudaFree(losses);
         cudaFreeHost(staged);
+        if (inputs_read) cudaEventDestroy(inputs_read);
     }
 };
 
@@ -700,6 +702,7 @@ int bine_mlp_create(int in_dim, int hidden, int out_dim, int max_batch, unsigned
     MLP_TRY(cudaMalloc(&m->losses, (nlosses + 1) * sizeof(float)));
     m->loss = m->losses + nlosses;
     MLP_TRY(cudaMallocHost(&m->staged, (off + 1) * sizeof(float)));
+    MLP_TRY(cudaEventCreateWithFlags(&m->inputs_read, cudaEventDisableTiming));
     MLP_TRY(cudaDeviceSynchronize());
     *out = m.release();
     return BINE_SUCCESS;
@@ -767,6 +770,9 @@ int bine_mlp_train_step(bine_mlp_t mlp, const float* d_x, const float* d_t, cons
     if (rc == BINE_SUCCESS) rc = prepare_batch(mlp, d_x, d_mask, n, s);
     if (rc) return rc;
     forward(mlp, n, nullptr, d_t, d_mask, s);
+    // The caller may refill or free its arrays on return, and only the stages
+    // up to here read them.
+    if (!loss) MLP_TRY(cudaEventRecord(mlp->inputs_read, s));
     backward(mlp, n, s);
     mlp->step++;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -777,6 +783,8 @@ int bine_mlp_train_step(bine_mlp_t mlp, const float* d_x, const float* d_t, cons
         MLP_TRY(cudaMemcpyAsync(mlp->staged + mlp->nparams, mlp->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
         MLP_TRY(cudaStreamSynchronize(s));
         *loss = mlp->staged[mlp->nparams];
+    } else {
+        MLP_TRY(cudaEventSynchronize(mlp->inputs_read));
     }
     MLP_TRY(cudaGetLastError());
     return BINE_SUCCESS;

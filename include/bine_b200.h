@@ -378,7 +378,10 @@ int bine_mlp_forward(bine_mlp_t mlp, const float *d_x, int n, float *d_y, void *
  * parameters), for checking against a CPU reference. */
 int bine_mlp_gradients(bine_mlp_t mlp, const float *d_x, const float *d_t, const float *d_mask, int n,
                        float *host_grads, float *loss);
-/* One Adam step on a batch; *loss receives the batch loss (synchronous). */
+/* One Adam step on a batch.  On return d_x, d_t and d_mask have been read and
+ * may be overwritten or freed.  With loss the whole step has ended and *loss
+ * holds the batch loss; with NULL the backward pass and the update may still
+ * be running on `stream`. */
 int bine_mlp_train_step(bine_mlp_t mlp, const float *d_x, const float *d_t, const float *d_mask, int n, float lr,
                         void *stream, float *loss);
 const char *bine_mlp_last_error(void);
