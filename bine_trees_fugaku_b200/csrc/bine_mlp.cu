@@ -546,6 +546,7 @@ struct bine_mlp_s {
     int* counts = nullptr;       // valid targets per prepare block
     float* losses = nullptr;     // loss per output tile, then the loss
     float* loss = nullptr;
+    float* side = nullptr;       // output, or targets and mask, where the caller's are not this device's
     float* staged = nullptr;     // pinned host copy of the gradients and the loss
     cudaEvent_t inputs_read = nullptr;  // a step's last read of the caller's arrays
     ~bine_mlp_s() {
@@ -560,6 +561,7 @@ struct bine_mlp_s {
         for (bf16* p : dpre) cudaFree(p);
         cudaFree(counts);
         cudaFree(losses);
+        cudaFree(side);
         cudaFreeHost(staged);
         if (inputs_read) cudaEventDestroy(inputs_read);
     }
@@ -570,21 +572,46 @@ namespace {
 int tiles(int n) { return (n + kTile - 1) / kTile; }
 
 // Rows of the batch (and the targets' mask, for a loss) to the layered path.
-int prepare_batch(bine_mlp_t mlp, const float* d_x, const float* d_mask, int n, cudaStream_t s) {
-    if (!mlp || !d_x || n <= 0 || n > mlp->max_batch || n % 16) return mfail(BINE_ERR_ARG, "batch must be a multiple of 16 within max_batch");
+void prepare_batch(bine_mlp_t mlp, const float* d_x, const float* d_mask, int n, cudaStream_t s) {
     k_prepare<<<kPrepBlocks, 256, 0, s>>>(d_x, mlp->x, (long long)n * mlp->din, d_mask, (long long)n * mlp->dout,
                                           mlp->counts);
+}
+
+// Whether kernels of the current device can work on a caller's array where it
+// is: its own and managed memory.  Memory of another device, which a kernel
+// reaches only with peer access, and pinned host memory go through `side` in
+// copies of the runtime.  Pageable memory is refused.
+int in_place(const float* p, bool* direct) {
+    cudaPointerAttributes at;
+    int dev = 0;
+    if (!p) return mfail(BINE_ERR_ARG, "null output, targets or mask");
+    MLP_TRY(cudaPointerGetAttributes(&at, p));
+    MLP_TRY(cudaGetDevice(&dev));
+    if (at.type == cudaMemoryTypeUnregistered)
+        return mfail(BINE_ERR_ARG, "output, targets and mask must be device arrays");
+    *direct = at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == dev);
     return BINE_SUCCESS;
 }
 
-// Targets and mask are read by the kernels where they are: device memory (or
-// host memory the device can reach).
-int check_targets(const float* d_t, const float* d_mask) {
-    for (const float* p : {d_t, d_mask}) {
-        cudaPointerAttributes at;
-        if (!p) return mfail(BINE_ERR_ARG, "null targets or mask");
-        MLP_TRY(cudaPointerGetAttributes(&at, p));
-        if (at.type == cudaMemoryTypeUnregistered) return mfail(BINE_ERR_ARG, "targets and mask must be device arrays");
+int check_batch(bine_mlp_t mlp, const float* d_x, int n) {
+    if (!mlp || !d_x || n <= 0 || n > mlp->max_batch || n % 16)
+        return mfail(BINE_ERR_ARG, "batch must be a multiple of 16 within max_batch");
+    return BINE_SUCCESS;
+}
+
+// Targets and mask as the kernels read them: *t and *mask are replaced by
+// their copies where needed.
+int place_targets(bine_mlp_t mlp, const float** t, const float** mask, int n, cudaStream_t s) {
+    bool direct[2];
+    int rc = in_place(*t, &direct[0]);
+    if (rc == BINE_SUCCESS) rc = in_place(*mask, &direct[1]);
+    if (rc) return rc;
+    const float** arr[2] = {t, mask};
+    for (int i = 0; i < 2; i++) {
+        if (direct[i]) continue;
+        float* own = mlp->side + (size_t)i * mlp->max_batch * mlp->dout;
+        MLP_TRY(cudaMemcpyAsync(own, *arr[i], sizeof(float) * (size_t)n * mlp->dout, cudaMemcpyDefault, s));
+        *arr[i] = own;
     }
     return BINE_SUCCESS;
 }
@@ -701,6 +728,7 @@ int bine_mlp_create(int in_dim, int hidden, int out_dim, int max_batch, unsigned
     const size_t nlosses = (size_t)tiles(max_batch) * tiles(out_dim);
     MLP_TRY(cudaMalloc(&m->losses, (nlosses + 1) * sizeof(float)));
     m->loss = m->losses + nlosses;
+    MLP_TRY(cudaMalloc(&m->side, 2 * (size_t)max_batch * out_dim * sizeof(float)));
     MLP_TRY(cudaMallocHost(&m->staged, (off + 1) * sizeof(float)));
     MLP_TRY(cudaEventCreateWithFlags(&m->inputs_read, cudaEventDisableTiming));
     MLP_TRY(cudaDeviceSynchronize());
@@ -735,10 +763,14 @@ int bine_mlp_set_params(bine_mlp_t mlp, const float* host) {
 
 int bine_mlp_forward(bine_mlp_t mlp, const float* d_x, int n, float* d_y, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    if (!d_y) return mfail(BINE_ERR_ARG, "null output");
-    int rc = prepare_batch(mlp, d_x, nullptr, n, s);
+    bool direct;
+    int rc = check_batch(mlp, d_x, n);
+    if (rc == BINE_SUCCESS) rc = in_place(d_y, &direct);
     if (rc) return rc;
-    forward(mlp, n, d_y, nullptr, nullptr, s);
+    prepare_batch(mlp, d_x, nullptr, n, s);
+    forward(mlp, n, direct ? d_y : mlp->side, nullptr, nullptr, s);
+    if (!direct)
+        MLP_TRY(cudaMemcpyAsync(d_y, mlp->side, sizeof(float) * (size_t)n * mlp->dout, cudaMemcpyDefault, s));
     MLP_TRY(cudaGetLastError());
     return BINE_SUCCESS;
 }
@@ -746,9 +778,10 @@ int bine_mlp_forward(bine_mlp_t mlp, const float* d_x, int n, float* d_y, void* 
 int bine_mlp_gradients(bine_mlp_t mlp, const float* d_x, const float* d_t, const float* d_mask, int n, float* host_grads,
                        float* loss) {
     cudaStream_t s = 0;
-    int rc = check_targets(d_t, d_mask);
-    if (rc == BINE_SUCCESS) rc = prepare_batch(mlp, d_x, d_mask, n, s);
+    int rc = check_batch(mlp, d_x, n);
+    if (rc == BINE_SUCCESS) rc = place_targets(mlp, &d_t, &d_mask, n, s);
     if (rc) return rc;
+    prepare_batch(mlp, d_x, d_mask, n, s);
     forward(mlp, n, nullptr, d_t, d_mask, s);
     backward(mlp, n, s);
     MLP_TRY(cudaGetLastError());
@@ -766,9 +799,10 @@ int bine_mlp_gradients(bine_mlp_t mlp, const float* d_x, const float* d_t, const
 int bine_mlp_train_step(bine_mlp_t mlp, const float* d_x, const float* d_t, const float* d_mask, int n, float lr,
                         void* stream, float* loss) {
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = check_targets(d_t, d_mask);
-    if (rc == BINE_SUCCESS) rc = prepare_batch(mlp, d_x, d_mask, n, s);
+    int rc = check_batch(mlp, d_x, n);
+    if (rc == BINE_SUCCESS) rc = place_targets(mlp, &d_t, &d_mask, n, s);
     if (rc) return rc;
+    prepare_batch(mlp, d_x, d_mask, n, s);
     forward(mlp, n, nullptr, d_t, d_mask, s);
     // The caller may refill or free its arrays on return, and only the stages
     // up to here read them.

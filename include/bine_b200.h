@@ -364,7 +364,9 @@ int bine_batch_autotune(const bine_batch_item_t *items, int nitems, void *stream
  * on timings and link-byte counts the engine itself measures and uses it to
  * choose variant, port count and segment size per call.  Not in the
  * reference.  All dimensions and batch sizes are multiples of 16; device
- * pointers are fp32 row-major [n x in] / [n x out]. */
+ * pointers are fp32 row-major [n x in] / [n x out].  Outputs, targets and
+ * masks may also be pinned host memory or memory of another device (they then
+ * go through copies); pageable memory is refused. */
 typedef struct bine_mlp_s *bine_mlp_t;
 int bine_mlp_create(int in_dim, int hidden, int out_dim, int max_batch, unsigned long long seed, bine_mlp_t *mlp);
 int bine_mlp_destroy(bine_mlp_t mlp);

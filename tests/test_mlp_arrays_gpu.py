@@ -41,3 +41,33 @@ def test_arrays_may_be_overwritten_after_a_step_without_a_loss(n, dout):
         assert np.array_equal(a.get_params(), b.get_params()), step
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,dout", [(16, 16), (48, 144)])
+def test_pinned_output_targets_and_mask(n, dout):
+    """Arrays that are not the device's own memory go through copies of the
+    runtime: the same bits as from device arrays."""
+    m = bine.MLP(16, 256, dout, 64, seed=6)
+    x, t, mask = batch(n, 16, dout, 1)
+    y = torch.full((n, dout), -1.0).pin_memory()
+    m._check(bine.lib().bine_mlp_forward(m._h, x.data_ptr(), n, y.data_ptr(), 0))
+    torch.cuda.synchronize()
+    assert torch.equal(y, m.forward(x).cpu())
+    g, loss = m.gradients(x, t, mask)
+    tp, mp = t.cpu().pin_memory(), mask.cpu().pin_memory()
+    for tt, mm in ((tp, mp), (tp, mask), (t, mp)):
+        g2, loss2 = m.gradients(x, tt, mm)
+        assert np.array_equal(g, g2) and loss == loss2
+    m.close()
+
+
+def test_a_pageable_output_is_refused():
+    """No kernel is launched on it."""
+    m = bine.MLP(16, 16, 16, 16)
+    x = torch.zeros((16, 16), device="cuda")
+    y = np.full((16, 16), -1.0, np.float32)
+    assert bine.lib().bine_mlp_forward(m._h, x.data_ptr(), 16, y.ctypes.data, 0) != bine.SUCCESS
+    assert bine.lib().bine_mlp_forward(m._h, x.data_ptr(), 16, None, 0) != bine.SUCCESS
+    torch.cuda.synchronize()
+    assert (y == -1).all()
+    m.close()
