@@ -229,11 +229,12 @@ struct ForwardArgs {
     float* losses;
     bf16* grad;
     int M, N, K;
+    int nx;  // tiles per row of tiles
 };
 __global__ void __launch_bounds__(kGemmThreads) k_forward(const ForwardArgs a) {
     __shared__ GemmSmem S;
     float acc[2][4];
-    const int row0 = blockIdx.y * kTile, col0 = blockIdx.x * kTile;
+    const int row0 = blockIdx.x / a.nx * kTile, col0 = blockIdx.x % a.nx * kTile;
     gemm_tile<false, false>(S, acc, a.in, a.K, a.w, a.K, row0, col0, a.M, a.N, a.K, [](const bf16*, int) {});
     if (a.act) {
         gemm_each(acc, row0, col0, a.M, a.N, [&](int r, int c, float v0, float v1) {
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_forward(const ForwardArgs a) {
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
         __syncthreads();
         if (threadIdx.x == 0)
-            a.losses[blockIdx.y * gridDim.x + blockIdx.x] = (part[0] + part[1] + part[2] + part[3]) * inv;
+            a.losses[blockIdx.x] = (part[0] + part[1] + part[2] + part[3]) * inv;
     }
 }
 
@@ -639,7 +640,10 @@ void forward(bine_mlp_t mlp, int n, float* d_y, const float* d_t, const float* d
             a.losses = mlp->losses;
             a.grad = mlp->dpre[l & 1];
         }
-        k_forward<<<dim3(tiles(a.N), tiles(n)), kGemmThreads, 0, s>>>(a);
+        // One row of the grid: a batch may have more rows of tiles than a
+        // grid has rows (65,535).
+        a.nx = tiles(a.N);
+        k_forward<<<(unsigned)(a.nx * tiles(n)), kGemmThreads, 0, s>>>(a);
     }
 }
 

@@ -71,3 +71,21 @@ def test_a_pageable_output_is_refused():
     torch.cuda.synchronize()
     assert (y == -1).all()
     m.close()
+
+
+def test_a_batch_of_more_rows_of_tiles_than_a_grid_has_rows():
+    """65,537 rows of 32-row tiles: the last rows are those of a small batch,
+    and the loss is the mean over all of them."""
+    n, last = 32 * 65537, 64
+    m = bine.MLP(16, 16, 16, n, seed=7)
+    x = torch.randn((n, 16), device="cuda")
+    y = m.forward(x)
+    assert torch.equal(y[-last:], m.forward(x[-last:].contiguous()))
+    assert torch.equal(y[:last], m.forward(x[:last].contiguous()))
+    t, mask = torch.zeros((n, 16), device="cuda"), torch.ones((n, 16), device="cuda")
+    g, loss = m.gradients(x, t, mask)
+    # 65,537 block partials in fp32, 2,049 to a lane, after the additions in
+    # a block: fewer than 4,200 in a row, each rounding by at most 2^-24.
+    assert abs(loss - float((y.double() ** 2).mean())) <= 4200 * 2.0 ** -24 * loss
+    assert np.isfinite(g).all()
+    m.close()
