@@ -297,6 +297,7 @@ struct bine_comm_s {
     int* status = nullptr;
     unsigned long long step_timeout_ns = 5ull * 1000 * 1000 * 1000;
     unsigned barrier_extra = 0;
+    size_t tree_smem_limit = 227 * 1024;  // static and dynamic, of a tree kernel's block
     // Host-buffer pipeline (bine_allreduce_host), created on first use:
     // copy streams, per-slot events (input copied, reduced, output copied)
     // and the device staging area (2 slots x input and output windows).
@@ -1078,132 +1079,130 @@ int get_dev_trees(bine_comm_t c, const PlanKey& k, int es, std::shared_ptr<DevTr
         return fail(BINE_ERR_CUDA, "uploading the reduction trees failed");
     // Split form: K lanes per output vector.
     if (K > 1) {
-        {
-            // K parts, one per warp, or 2K parts assigned longest first when
-            // that lowers the busiest warp's leaves by 5 % or more (trees of
-            // non-power-of-two P do not cut into K equal subtrees).
-            auto lpt = [&](const SplitTrees& t, int np, size_t seg, std::vector<std::vector<int>>* mine) {
-                const int32_t* po = &t.parts[seg * (np + 1)];
-                std::vector<int> order(np), load(K, 0);
-                mine->assign(K, {});
-                for (int j = 0; j < np; j++) order[j] = j;
-                std::stable_sort(order.begin(), order.end(),
-                                 [&](int x, int y) { return po[x + 1] - po[x] > po[y + 1] - po[y]; });
-                for (int p : order) {
-                    const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-                    (*mine)[w].push_back(p);
-                    load[w] += po[p + 1] - po[p];
-                }
-                return *std::max_element(load.begin(), load.end());
-            };
-            SplitTrees s1, s2;
-            if (!split_trees(tp, K, &s1, &err) || !split_trees(tp, 2 * K, &s2, &err)) return fail(BINE_ERR_INTERNAL, err);
-            long long max1 = 0, max2 = 0;
-            std::vector<std::vector<int>> tmp;
-            for (size_t i = 0; i < tp.segs.size(); i++) {
-                max1 += lpt(s1, K, i, &tmp);
-                max2 += lpt(s2, 2 * K, i, &tmp);
+        // K parts, one per warp, or 2K parts assigned longest first when
+        // that lowers the busiest warp's leaves by 5 % or more (trees of
+        // non-power-of-two P do not cut into K equal subtrees).
+        auto lpt = [&](const SplitTrees& t, int np, size_t seg, std::vector<std::vector<int>>* mine) {
+            const int32_t* po = &t.parts[seg * (np + 1)];
+            std::vector<int> order(np), load(K, 0);
+            mine->assign(K, {});
+            for (int j = 0; j < np; j++) order[j] = j;
+            std::stable_sort(order.begin(), order.end(),
+                             [&](int x, int y) { return po[x + 1] - po[x] > po[y + 1] - po[y]; });
+            for (int p : order) {
+                const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+                (*mine)[w].push_back(p);
+                load[w] += po[p + 1] - po[p];
             }
-            const bool two = max2 * 100 <= max1 * 95;
-            const SplitTrees& st = two ? s2 : s1;
-            const int KP = two ? 2 * K : K;
-            if (st.max_depth > dev::kMaxTreeDepth) return fail(BINE_ERR_UNSUPPORTED, "reduction tree deeper than supported");
-            std::vector<dev::TreeSeg> ssegs;
-            std::vector<int> sparts, sassign;
-            std::vector<dev::TreeComb> scomb;
-            std::vector<dev::TreeTile> stiles;
-            for (size_t i = 0; i < tp.segs.size(); i++) {
-                const OutSegment& sg = tp.segs[i];
-                const int32_t* po = &st.parts[i * (KP + 1)];
-                const int32_t b = po[0], e = po[KP];
-                ssegs.push_back(dev::TreeSeg{sg.off, sg.n, sg.rank, b, e - b, sg.depth});
-                d->smax_prog_len = std::max(d->smax_prog_len, e - b);
-                for (int j = 0; j <= KP; j++) sparts.push_back(po[j] - b);
-                for (int j = 0; j < KP; j++) scomb.push_back(dev::TreeComb{st.comb[i * KP + j].first, st.comb[i * KP + j].second});
-                std::vector<std::vector<int>> mine;
-                lpt(st, KP, i, &mine);
-                std::vector<int> offs{0};
-                for (int w = 0; w < K; w++) {
-                    sassign.insert(sassign.end(), mine[w].begin(), mine[w].end());
-                    offs.push_back(offs.back() + (int)mine[w].size());
-                }
-                sassign.insert(sassign.end(), offs.begin(), offs.end());
-                add_tiles(&stiles, (int32_t)i, body_lo[i], body_hi[i], (int64_t)(dev::kThreads / K) * L);
-            }
-            d->split_parts = KP;
-            FlatTables ft;
-            SplitTrees se;
-            std::string serr;
-            const bool have_se = min_leaves >= 2 * dev::kEdgeParts && split_trees(tp, dev::kEdgeParts, &se, &serr) &&
-                                 se.max_depth <= dev::kMaxTreeDepth;
-            if (flat_tables(tp, st, have_se ? &se : nullptr, K, KP, sassign, body_lo, body_hi,
-                            (int64_t)(dev::kThreads / K) * L, (int)L, c->P, &ft)) {
-                cudaError_t g[9];
-                put(&d->fbody, ft.body, &g[0]);
-                put(&d->franks, ft.ranks, &g[1]);
-                put(&d->feshape, ft.eshape, &g[2]);
-                put(&d->fadds, ft.adds, &g[3]);
-                put(&d->fparts, ft.parts, &g[4]);
-                put(&d->fcomb, ft.comb, &g[5]);
-                put(&d->fassign, ft.assign, &g[6]);
-                put(&d->fedges, ft.edges, &g[7]);
-                cudaError_t h[4];
-                put(&d->feadds, ft.eadds, &h[0]);
-                put(&d->feparts, ft.eparts, &h[1]);
-                put(&d->fecomb, ft.ecomb, &h[2]);
-                put(&d->feranks_t, ft.eranks_t, &h[3]);
-                for (cudaError_t x : h)
-                    if (x != cudaSuccess) return fail(BINE_ERR_CUDA, "uploading the row-aligned reduction trees failed");
-                d->nfedges = (int)ft.edges.size();
-                d->felen = ft.len;
-                d->fedepth = ft.edepth;
-                // The element kernel keeps only the pieces no edge covers.
-                std::vector<dev::TreeTile> keep;
-                for (const dev::TreeTile& t : htiles)
-                    if (!ft.covered.count({t.seg, t.start})) keep.push_back(t);
-                if (!dry) cudaFree(d->htiles);
-                d->htiles = nullptr;
-                put(&d->htiles, keep, &g[8]);
-                for (cudaError_t x : g)
-                    if (x != cudaSuccess) return fail(BINE_ERR_CUDA, "uploading the row-aligned reduction trees failed");
-                d->nhtiles = (int)keep.size();
-                d->h_htiles = keep;
-                d->flat = true;
-                d->fpitch = ft.pitch;
-                d->flen = ft.len;
-                d->fmax_ns = ft.max_ns;
-                d->fnq = ft.nq;
-                d->fnshape = ft.nshape;
-                d->h_fedges = ft.edges;
-                d->h_fbody = ft.body;
-                stiles = std::move(ft.tiles);
-            }
-            std::vector<dev::TreeEntry> sprog;
-            for (const ProgEntry& e : st.prog) sprog.push_back(dev::TreeEntry{e.rank, e.adds, e.shift});
-            cudaError_t f1, f2, f3, f4, f5, f6;
-            put(&d->ssegs, ssegs, &f1);
-            put(&d->sprog, sprog, &f2);
-            put(&d->sparts, sparts, &f3);
-            put(&d->scomb, scomb, &f4);
-            put(&d->stiles, stiles, &f5);
-            put(&d->sassign, sassign, &f6);
-            if (f1 != cudaSuccess || f2 != cudaSuccess || f3 != cudaSuccess || f4 != cudaSuccess || f5 != cudaSuccess ||
-                f6 != cudaSuccess)
-                return fail(BINE_ERR_CUDA, "uploading the split reduction trees failed");
-            d->nstiles = (int)stiles.size();
-            // Stack slots: the deepest part program or combine program.
-            int cdepth = 1;
-            for (size_t q = 0; q < st.comb.size(); q += KP) {
-                int sp = 0;
-                for (int j = 0; j < KP; j++) {
-                    cdepth = std::max(cdepth, ++sp);
-                    sp -= st.comb[q + j].second;
-                }
-            }
-            d->sdepth = std::max(st.max_depth, cdepth);
-            d->h_stiles = stiles;
-            d->split_k = K;
+            return *std::max_element(load.begin(), load.end());
+        };
+        SplitTrees s1, s2;
+        if (!split_trees(tp, K, &s1, &err) || !split_trees(tp, 2 * K, &s2, &err)) return fail(BINE_ERR_INTERNAL, err);
+        long long max1 = 0, max2 = 0;
+        std::vector<std::vector<int>> tmp;
+        for (size_t i = 0; i < tp.segs.size(); i++) {
+            max1 += lpt(s1, K, i, &tmp);
+            max2 += lpt(s2, 2 * K, i, &tmp);
         }
+        const bool two = max2 * 100 <= max1 * 95;
+        const SplitTrees& st = two ? s2 : s1;
+        const int KP = two ? 2 * K : K;
+        if (st.max_depth > dev::kMaxTreeDepth) return fail(BINE_ERR_UNSUPPORTED, "reduction tree deeper than supported");
+        std::vector<dev::TreeSeg> ssegs;
+        std::vector<int> sparts, sassign;
+        std::vector<dev::TreeComb> scomb;
+        std::vector<dev::TreeTile> stiles;
+        for (size_t i = 0; i < tp.segs.size(); i++) {
+            const OutSegment& sg = tp.segs[i];
+            const int32_t* po = &st.parts[i * (KP + 1)];
+            const int32_t b = po[0], e = po[KP];
+            ssegs.push_back(dev::TreeSeg{sg.off, sg.n, sg.rank, b, e - b, sg.depth});
+            d->smax_prog_len = std::max(d->smax_prog_len, e - b);
+            for (int j = 0; j <= KP; j++) sparts.push_back(po[j] - b);
+            for (int j = 0; j < KP; j++) scomb.push_back(dev::TreeComb{st.comb[i * KP + j].first, st.comb[i * KP + j].second});
+            std::vector<std::vector<int>> mine;
+            lpt(st, KP, i, &mine);
+            std::vector<int> offs{0};
+            for (int w = 0; w < K; w++) {
+                sassign.insert(sassign.end(), mine[w].begin(), mine[w].end());
+                offs.push_back(offs.back() + (int)mine[w].size());
+            }
+            sassign.insert(sassign.end(), offs.begin(), offs.end());
+            add_tiles(&stiles, (int32_t)i, body_lo[i], body_hi[i], (int64_t)(dev::kThreads / K) * L);
+        }
+        d->split_parts = KP;
+        FlatTables ft;
+        SplitTrees se;
+        std::string serr;
+        const bool have_se = min_leaves >= 2 * dev::kEdgeParts && split_trees(tp, dev::kEdgeParts, &se, &serr) &&
+                             se.max_depth <= dev::kMaxTreeDepth;
+        if (flat_tables(tp, st, have_se ? &se : nullptr, K, KP, sassign, body_lo, body_hi,
+                        (int64_t)(dev::kThreads / K) * L, (int)L, c->P, &ft)) {
+            cudaError_t g[9];
+            put(&d->fbody, ft.body, &g[0]);
+            put(&d->franks, ft.ranks, &g[1]);
+            put(&d->feshape, ft.eshape, &g[2]);
+            put(&d->fadds, ft.adds, &g[3]);
+            put(&d->fparts, ft.parts, &g[4]);
+            put(&d->fcomb, ft.comb, &g[5]);
+            put(&d->fassign, ft.assign, &g[6]);
+            put(&d->fedges, ft.edges, &g[7]);
+            cudaError_t h[4];
+            put(&d->feadds, ft.eadds, &h[0]);
+            put(&d->feparts, ft.eparts, &h[1]);
+            put(&d->fecomb, ft.ecomb, &h[2]);
+            put(&d->feranks_t, ft.eranks_t, &h[3]);
+            for (cudaError_t x : h)
+                if (x != cudaSuccess) return fail(BINE_ERR_CUDA, "uploading the row-aligned reduction trees failed");
+            d->nfedges = (int)ft.edges.size();
+            d->felen = ft.len;
+            d->fedepth = ft.edepth;
+            // The element kernel keeps only the pieces no edge covers.
+            std::vector<dev::TreeTile> keep;
+            for (const dev::TreeTile& t : htiles)
+                if (!ft.covered.count({t.seg, t.start})) keep.push_back(t);
+            if (!dry) cudaFree(d->htiles);
+            d->htiles = nullptr;
+            put(&d->htiles, keep, &g[8]);
+            for (cudaError_t x : g)
+                if (x != cudaSuccess) return fail(BINE_ERR_CUDA, "uploading the row-aligned reduction trees failed");
+            d->nhtiles = (int)keep.size();
+            d->h_htiles = keep;
+            d->flat = true;
+            d->fpitch = ft.pitch;
+            d->flen = ft.len;
+            d->fmax_ns = ft.max_ns;
+            d->fnq = ft.nq;
+            d->fnshape = ft.nshape;
+            d->h_fedges = ft.edges;
+            d->h_fbody = ft.body;
+            stiles = std::move(ft.tiles);
+        }
+        std::vector<dev::TreeEntry> sprog;
+        for (const ProgEntry& e : st.prog) sprog.push_back(dev::TreeEntry{e.rank, e.adds, e.shift});
+        cudaError_t f1, f2, f3, f4, f5, f6;
+        put(&d->ssegs, ssegs, &f1);
+        put(&d->sprog, sprog, &f2);
+        put(&d->sparts, sparts, &f3);
+        put(&d->scomb, scomb, &f4);
+        put(&d->stiles, stiles, &f5);
+        put(&d->sassign, sassign, &f6);
+        if (f1 != cudaSuccess || f2 != cudaSuccess || f3 != cudaSuccess || f4 != cudaSuccess || f5 != cudaSuccess ||
+            f6 != cudaSuccess)
+            return fail(BINE_ERR_CUDA, "uploading the split reduction trees failed");
+        d->nstiles = (int)stiles.size();
+        // Stack slots: the deepest part program or combine program.
+        int cdepth = 1;
+        for (size_t q = 0; q < st.comb.size(); q += KP) {
+            int sp = 0;
+            for (int j = 0; j < KP; j++) {
+                cdepth = std::max(cdepth, ++sp);
+                sp -= st.comb[q + j].second;
+            }
+        }
+        d->sdepth = std::max(st.max_depth, cdepth);
+        d->h_stiles = stiles;
+        d->split_k = K;
     }
     if (dry) {
         *out = d;
@@ -1335,23 +1334,34 @@ struct TreeSmem {
     int stack_off;  // in 16-byte words
     bool stack;
 };
-TreeSmem tree_smem(int prog_len, int depth) {
+TreeSmem tree_smem(bine_comm_t c, int prog_len, int depth) {
     static_assert(sizeof(dev::TreeEntry) == 16, "program entries are 16-byte words");
     const size_t prog = (size_t)std::max(1, prog_len) * 16;
     const size_t stack = (size_t)std::max(1, depth) * dev::kThreads * 16;
-    const bool in_smem = stack <= 64 * 1024 && prog + stack <= 200 * 1024;
+    // 27 KB for the kernels' static tables.
+    const bool in_smem = stack <= 64 * 1024 && prog + stack + 27 * 1024 <= c->tree_smem_limit;
     return TreeSmem{prog + (in_smem ? stack : 0), (int)(prog / 16), in_smem};
+}
+
+// Static and dynamic shared memory of a block of `kern`.
+template <typename K>
+int total_smem(K kern, size_t smem, size_t* total) {
+    cudaFuncAttributes fa;
+    CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
+    *total = smem + fa.sharedSizeBytes;
+    return BINE_SUCCESS;
 }
 
 template <typename K>
 int launch_tree_kernel(bine_comm_t c, K kern, size_t smem, long long ntiles, unsigned* grid) {
-    // Static and dynamic shared memory together: above 48 KB the dynamic
-    // part needs the opt-in attribute, above 227 KB it cannot launch.
-    cudaFuncAttributes fa;
-    CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
-    if (smem + fa.sharedSizeBytes > 227 * 1024)
+    // Above 48 KB the dynamic part needs the opt-in attribute, above 227 KB
+    // together the kernel cannot launch.
+    size_t total;
+    int rc = total_smem(kern, smem, &total);
+    if (rc) return rc;
+    if (total > c->tree_smem_limit)
         return fail(BINE_ERR_UNSUPPORTED, "reduction program does not fit in shared memory");
-    if (smem + fa.sharedSizeBytes > 48 * 1024)
+    if (total > 48 * 1024)
         CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // One block per tile, up to 64 blocks per SM (then grid-stride): the
     // hardware back-fills SMs as blocks finish.  Measured on B200 against a
@@ -1365,7 +1375,7 @@ template <typename T, int K>
 int launch_tree_split(bine_comm_t c, const DevTrees& d, const char* in, long long ist, char* out, long long ost,
                       const dev::TreeTile* stiles, int nstiles) {
     if (nstiles == 0) return BINE_SUCCESS;
-    const TreeSmem sm = tree_smem(d.smax_prog_len, d.sdepth);
+    const TreeSmem sm = tree_smem(c, d.smax_prog_len, d.sdepth);
     auto kern = sm.stack ? dev::k_tree_split<T, K, true> : dev::k_tree_split<T, K, false>;
     unsigned g = 0;
     int rc = launch_tree_kernel(c, kern, sm.bytes, nstiles, &g);
@@ -1382,14 +1392,17 @@ template <typename T, int K>
 int launch_tree_strided(bine_comm_t c, const DevTrees& d, const char* in, long long ist, char* out, long long ost,
                         const dev::TreeTile* tiles, int ntiles, cudaStream_t s) {
     const bool split = K > 1;
-    const TreeSmem sm = tree_smem(split ? d.smax_prog_len : d.max_prog_len, split ? d.sdepth : d.depth);
+    const TreeSmem sm = tree_smem(c, split ? d.smax_prog_len : d.max_prog_len, split ? d.sdepth : d.depth);
     auto kern = sm.stack ? dev::k_tree_strided<T, K, true> : dev::k_tree_strided<T, K, false>;
-    unsigned g = 0;
-    int rc = launch_tree_kernel(c, kern, sm.bytes, ntiles, &g);
     if constexpr (K > 1) {
         // The largest programs leave no room for the parts' partial sums.
-        if (rc == BINE_ERR_UNSUPPORTED) return launch_tree_strided<T, 1>(c, d, in, ist, out, ost, tiles, ntiles, s);
+        size_t total;
+        int rc = total_smem(kern, sm.bytes, &total);
+        if (rc) return rc;
+        if (total > c->tree_smem_limit) return launch_tree_strided<T, 1>(c, d, in, ist, out, ost, tiles, ntiles, s);
     }
+    unsigned g = 0;
+    int rc = launch_tree_kernel(c, kern, sm.bytes, ntiles, &g);
     if (rc) return rc;
     kern<<<g, dev::kThreads, sm.bytes, s>>>(in, ist, out, ost, c->P, split ? d.ssegs : d.segs,
                                             split ? d.sprog : d.prog, d.sparts, d.scomb, d.sassign, tiles, ntiles,
@@ -1558,7 +1571,7 @@ int launch_tree(bine_comm_t c, const DevTrees& d, const char* in, long long ist,
         }
         if (rc) return rc;
     } else if (vec && ts.n[0] > 0) {
-        const TreeSmem sm = tree_smem(d.max_prog_len, d.depth);
+        const TreeSmem sm = tree_smem(c, d.max_prog_len, d.depth);
         auto kern = sm.stack ? dev::k_tree_vec<T, true> : dev::k_tree_vec<T, false>;
         rc = launch_tree_kernel(c, kern, sm.bytes, ts.n[0], &g);
         if (rc) return rc;
@@ -2764,6 +2777,12 @@ int bine_comm_set_step_timeout(bine_comm_t comm, unsigned timeout_ms) {
 int bine_debug_set_barrier_extra(bine_comm_t comm, unsigned extra) {
     if (!comm) return fail(BINE_ERR_ARG, "null communicator");
     comm->barrier_extra = extra;
+    return BINE_SUCCESS;
+}
+
+int bine_debug_set_tree_smem_limit(bine_comm_t comm, size_t bytes) {
+    if (!comm || bytes > 227 * 1024) return fail(BINE_ERR_ARG, "the limit is at most 227 KB");
+    comm->tree_smem_limit = bytes;
     return BINE_SUCCESS;
 }
 

@@ -276,6 +276,11 @@ int bine_comm_set_step_timeout(bine_comm_t comm, unsigned timeout_ms);
  * faults or hangs. */
 int bine_debug_set_barrier_extra(bine_comm_t comm, unsigned extra);
 
+/* Debug: shared memory that a block of an exact-order float kernel may use
+ * (at most 227 KB, the default), so that small calls reach what large
+ * reduction programs do. */
+int bine_debug_set_tree_smem_limit(bine_comm_t comm, size_t bytes);
+
 /* How the FUSED engine evaluates an exact-order float reduction on a
  * 16-byte-aligned layout, planned on the host only (no device needed;
  * nothing is uploaded or cached):
