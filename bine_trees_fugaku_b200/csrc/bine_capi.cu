@@ -2343,7 +2343,7 @@ int noalloc_run(bine_comm_t c, const Schedule& s, const char* send, long long is
 // ---------------------------------------------------------------- batches
 struct bine_batch_s {
     dev::BatchItem* items = nullptr;
-    int* hint = nullptr;  // call of every kBatchHint-th tile, then the last call
+    int* hint = nullptr;  // call of every kBatchHint-th tile, then the last call; null: search all calls
     int nitems = 0;
     long long total_tiles = 0;
     unsigned grid = 1;
@@ -2437,7 +2437,7 @@ unsigned batch_grid(long long total_tiles, int grid_mult) {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_batch, dev::kThreads, 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_batch<true>, dev::kThreads, 0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     long long g = (long long)per_sm * sms * std::max(1, grid_mult);
     return (unsigned)std::max(1LL, std::min(g, total_tiles));
@@ -2463,16 +2463,19 @@ int bine_batch_create(const bine_batch_item_t* items, int nitems, const bine_bat
     if (!v.empty()) {
         CUDA_TRY(cudaMalloc(&b->items, v.size() * sizeof(dev::BatchItem)));
         CUDA_TRY(cudaMemcpy(b->items, v.data(), v.size() * sizeof(dev::BatchItem), cudaMemcpyHostToDevice));
-        std::vector<int> hint;
-        int k = 0;
-        for (long long t = 0; t < tiles; t += dev::kBatchHint) {
-            while (k + 1 < (int)v.size() && v[k + 1].tile_begin <= t) k++;
-            hint.push_back(k);
+        // Up to kBatchHint tiles the table has one range, of all the calls.
+        if (tiles > dev::kBatchHint) {
+            std::vector<int> hint;
+            int k = 0;
+            for (long long t = 0; t < tiles; t += dev::kBatchHint) {
+                while (k + 1 < (int)v.size() && v[k + 1].tile_begin <= t) k++;
+                hint.push_back(k);
+            }
+            hint.push_back((int)v.size() - 1);
+            cudaError_t e;
+            fill(&b->hint, hint, &e);
+            if (e != cudaSuccess) return fail(BINE_ERR_CUDA, "uploading the batch failed");
         }
-        hint.push_back((int)v.size() - 1);
-        cudaError_t e;
-        fill(&b->hint, hint, &e);
-        if (e != cudaSuccess) return fail(BINE_ERR_CUDA, "uploading the batch failed");
     }
     *batch = b.release();
     return BINE_SUCCESS;
@@ -2481,7 +2484,9 @@ int bine_batch_create(const bine_batch_item_t* items, int nitems, const bine_bat
 int bine_batch_launch(bine_batch_t batch, void* stream) {
     if (!batch) return fail(BINE_ERR_ARG, "null batch");
     if (batch->total_tiles == 0) return BINE_SUCCESS;
-    dev::k_batch<<<batch->grid, dev::kThreads, 0, (cudaStream_t)stream>>>(batch->items, batch->hint, batch->total_tiles);
+    auto kern = batch->hint ? dev::k_batch<true> : dev::k_batch<false>;
+    kern<<<batch->grid, dev::kThreads, 0, (cudaStream_t)stream>>>(batch->items, batch->nitems, batch->hint,
+                                                                  batch->total_tiles);
     CUDA_TRY(cudaGetLastError());
     return BINE_SUCCESS;
 }

@@ -2337,7 +2337,10 @@ __global__ void k_link_scan(Torus t, unsigned long long* links) {
 // different P, sizes and element types in ONE launch.  Every call is cut
 // into tiles; blocks take tiles grid-stride from the global tile range and
 // find their call by a binary search over tile_begin, bounded by a table of
-// the calls at every kBatchHint-th tile.  Reduction tiles are `tc` 16-byte
+// the calls at every kBatchHint-th tile (no table up to kBatchHint tiles,
+// where it holds one range: a small call with its data outside L2 takes 6.1
+// us, 8.2 with the table's dependent load; both forms in one kernel cost
+// batches of 100 calls 2 us).  Reduction tiles are `tc` 16-byte
 // columns wide and split the P rows over 256/tc row groups (tc comes from
 // the tuning: narrow tiles with many row groups for large P, wide tiles for
 // small P); allgather tiles are 256 vectors of the flattened (source rank,
@@ -2414,12 +2417,13 @@ __device__ __forceinline__ void batch_reduce_tile(const BatchItem& it, long long
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_batch(const BatchItem* __restrict__ items,
-                                                       const int* __restrict__ hint, long long total_tiles) {
+template <bool TABLE>
+__global__ void __launch_bounds__(kThreads) k_batch(const BatchItem* __restrict__ items, int nitems,
+                                                    const int* __restrict__ hint, long long total_tiles) {
     __shared__ Lanes<float, double> part[kThreads];
     __shared__ uint4 res[kThreads];
     for (long long t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        int lo = hint[t / kBatchHint], hi = hint[t / kBatchHint + 1];
+        int lo = TABLE ? hint[t / kBatchHint] : 0, hi = TABLE ? hint[t / kBatchHint + 1] : nitems - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) / 2;
             if (items[mid].tile_begin <= t) lo = mid;
