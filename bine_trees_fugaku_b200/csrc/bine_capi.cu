@@ -1297,7 +1297,13 @@ int launch_sum(bine_comm_t c, int mode, const char* in, long long ist, char* out
     }
     const long long rest = elems - done;
     if (rest == 0) return BINE_SUCCESS;
-    if constexpr (sizeof(T) == 1) {
+    // One element per thread for 1-byte elements and below 16 ranks, where a
+    // strided lane vector gains nothing over its longer chain (us, strided /
+    // per element, int32 allreduce: P = 4, 1 element 1.95 / 1.73; P = 8, 20,001
+    // 2.88 / 2.59; P = 12, 300,001 5.95 / 5.66; float32 in the FAST order, P = 9,
+    // 672,944 12.4 / 8.3).  At P = 16 the two are equal for rows in L2 and the
+    // vectors 10 % faster for rows outside it.
+    if (sizeof(T) == 1 || c->P < 16) {
         const unsigned g = grid_for(c, rest);
         if (mode == dev::kSumAllreduce)
             dev::k_sum_scalar<T, dev::kSumAllreduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, c->P, done, rest, blk, root);
@@ -1307,11 +1313,13 @@ int launch_sum(bine_comm_t c, int mode, const char* in, long long ist, char* out
             dev::k_sum_scalar<T, dev::kSumReduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, c->P, done, rest, blk, root);
         CUDA_TRY(cudaGetLastError());
         return BINE_SUCCESS;
-    } else {
+    }
+    if constexpr (sizeof(T) > 1) {
         const long long off = done * es;
         return launch_sum_range<T, false>(c, mode, in + off, ist, mode == dev::kSumReduceScatter ? out : out + off,
                                           ost, rest, blk, root, done);
     }
+    return BINE_SUCCESS;
 }
 
 int launch_sum_dt(bine_comm_t c, int dt, int mode, const char* in, long long ist, char* out, long long ost,

@@ -274,10 +274,11 @@ __global__ void __launch_bounds__(kThreads) k_sum_vec(const char* __restrict__ i
     }
 }
 
-// Sums of 1-byte elements off the 16-byte grid, elements [e0, e0 + n) of
-// every row, one per thread: a strided lane vector would take 16 loads of
-// one byte each (int8 allreduce at P = 96, 262,147 elements per rank: 20.7 us
-// here, 33.3 us strided).  reduce_scatter: `blk` elements per rank.
+// Sums off the 16-byte grid of 1-byte elements and of fewer than 16 ranks,
+// elements [e0, e0 + n) of every row, one per thread: a strided lane vector of
+// bytes would take 16 loads of one byte each (int8 allreduce at P = 96,
+// 262,147 elements per rank: 20.7 us here, 33.3 us strided), and with few rows
+// one thread's loads are few.  reduce_scatter: `blk` elements per rank.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kThreads) k_sum_scalar(const char* __restrict__ in, long long in_stride,
                                                          char* __restrict__ out, long long out_stride, int P,

@@ -1,0 +1,28 @@
+"""Calls on either side of the lines between the kernels for rows and blocks
+off the 16-byte grid, against exact sums and copies."""
+import numpy as np
+import pytest
+
+import bine_trees_fugaku_b200 as bine
+from oracle.common import buffer_counts, expected
+from tests.test_ragged_gpu import call, values
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("coll", ["allreduce", "reduce", "reduce_scatter"])
+@pytest.mark.parametrize("P", [15, 16])
+@pytest.mark.parametrize("count,shift,pad", [(1, 0, 0), (1027, 1, 0), (1026, 0, 2)])
+def test_sums_below_and_from_16_ranks(coll, P, count, shift, pad):
+    """One element per thread below 16 ranks, strided vectors from there on;
+    float32 in the FAST order: FP64 accumulation and one rounding, within half
+    an ulp of the FP64 sum and that sum's own P 2^-52 sum|x|."""
+    si, _ = buffer_counts(coll, count, P)
+    rows = [0] if coll == "reduce" else slice(None)
+    x = values((P, si), np.int64, P + count)
+    assert np.array_equal(call(coll, x, count, shift, pad)[rows], expected(coll, x, P, count, 0)[rows])
+    x = values((P, si), np.float32, P + count)
+    want = expected(coll, x.astype(np.float64), P, count, 0)[rows]
+    absum = expected(coll, np.abs(x).astype(np.float64), P, count, 0)[rows]
+    got = call(coll, x, count, shift, pad, order="fast")[rows]
+    assert np.all(np.abs(got - want) <= np.abs(want) * 2.0 ** -24 + P * 2.0 ** -52 * absum)
