@@ -1257,7 +1257,7 @@ int launch_sum_cols(bine_comm_t c, int mode, const char* in, long long ist, char
 }
 
 // Sums of elements [e0, e0 + n) of every row (`in` and, except for
-// reduce_scatter, `out` point at element e0).
+// reduce_scatter, `out` point at element e0); `blk` as k_sum_vec takes it.
 template <typename T, bool VEC>
 int launch_sum_range(bine_comm_t c, int mode, const char* in, long long ist, char* out, long long ost, long long n,
                      long long blk, int root, long long e0) {
@@ -1292,7 +1292,7 @@ int launch_sum(bine_comm_t c, int mode, const char* in, long long ist, char* out
                      (mode != dev::kSumReduceScatter || (blk * es) % 16 == 0);
     const long long done = vec ? elems * es / 16 * (16 / es) : 0;
     if (done > 0) {
-        int rc = launch_sum_range<T, true>(c, mode, in, ist, out, ost, done, blk, root, 0);
+        int rc = launch_sum_range<T, true>(c, mode, in, ist, out, ost, done, blk * es / 16, root, 0);
         if (rc) return rc;
     }
     const long long rest = elems - done;

@@ -26,3 +26,13 @@ def test_sums_below_and_from_16_ranks(coll, P, count, shift, pad):
     absum = expected(coll, np.abs(x).astype(np.float64), P, count, 0)[rows]
     got = call(coll, x, count, shift, pad, order="fast")[rows]
     assert np.all(np.abs(got - want) <= np.abs(want) * 2.0 ** -24 + P * 2.0 ** -52 * absum)
+
+
+@pytest.mark.parametrize("dtype", [np.int8, np.int32, np.int64, np.float64])
+@pytest.mark.parametrize("P,vectors", [(2, 1), (17, 1), (768, 1), (64, 16), (5, 1031)])
+def test_reduce_scatter_of_whole_vectors(P, vectors, dtype):
+    """Blocks of one vector to several tiles on the 16-byte grid: every vector
+    at its owner's place."""
+    count = vectors * 16 // np.dtype(dtype).itemsize
+    x = values((P, P * count), np.int8, P + vectors).astype(dtype)
+    assert np.array_equal(call("reduce_scatter", x, count, pad=0, order="fast"), expected("reduce_scatter", x, P, count))
