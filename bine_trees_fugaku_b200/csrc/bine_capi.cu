@@ -1639,7 +1639,13 @@ int launch_copy_units(bine_comm_t c, int mode, dev::CopyArgs a) {
             }
         }
     }
-    if (!spread && nu >= dev::kCopyBlockMin) {
+    // Calls of up to kCopySmallMax elements leave threads idle: with one
+    // element per thread none of them waits for a second load (us, pieces or
+    // realigned vectors / one element: scatter at P = 32 of 192 float32 2.69 /
+    // 2.40, of 1,200 2.30 / 2.05, of 400 off the grid 3.20 / 2.05; alltoall at
+    // P = 4 of 400 off the grid 3.10 / 2.08).  At 303,104 elements, one per
+    // thread that the GPU holds, vectors on the grid lose again.
+    if (!spread && nu >= dev::kCopyBlockMin && units > dev::kCopySmallMax) {
         // Realigned vectors for 4-byte elements from 1 KiB per block and for
         // narrower ones from 256 bytes; elements otherwise (us, elements /
         // realigned: alltoall at P = 256 with 516-byte blocks 25 / 45, with

@@ -1077,9 +1077,11 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_copy_rows(CopyArg
     }
 }
 
-// Blocks of fewer than kCopyBlockMin elements with one destination: four
-// elements per thread and round, over the elements of all blocks in order
-// (I: the index type, 32 bits where the element count allows).
+// Blocks of fewer than kCopyBlockMin elements with one destination, and calls
+// of at most kCopySmallMax: up to four elements per thread and round, over
+// the elements of all blocks in order (I: the index type, 32 bits where the
+// element count allows), as many threads as elements where the grid holds them.
+constexpr int kCopySmallMax = 65536;
 template <int MODE, typename U, typename I>
 __global__ void __launch_bounds__(kThreads) k_copy_small(CopyArgs a) {
     const I nu = (I)(a.unit / (long long)sizeof(U)), P = (I)a.P;

@@ -36,3 +36,17 @@ def test_reduce_scatter_of_whole_vectors(P, vectors, dtype):
     count = vectors * 16 // np.dtype(dtype).itemsize
     x = values((P, P * count), np.int8, P + vectors).astype(dtype)
     assert np.array_equal(call("reduce_scatter", x, count, pad=0, order="fast"), expected("reduce_scatter", x, P, count))
+
+
+@pytest.mark.parametrize("dtype,count,shift", [
+    (np.int8, 1021, 1), (np.int8, 1024, 0), (np.int8, 1040, 0), (np.int32, 1024, 1), (np.int32, 1031, 0), (np.int32, 4096, 0),
+    (np.int32, 4100, 0), (np.int64, 1024, 1), (np.int64, 1025, 0)])
+@pytest.mark.parametrize("coll,P", [("scatter", 64), ("gather", 64), ("alltoall", 8)])
+def test_block_copies_around_65536_elements(coll, P, dtype, count, shift):
+    """64 blocks each: at and below 65,536 elements of the widest type that
+    fits the call one per thread, above pieces or realigned vectors."""
+    root = P - 1
+    si, _ = buffer_counts(coll, count, P)
+    x = values((P, si), dtype, count)
+    rows = [root] if coll == "gather" else slice(None)
+    assert np.array_equal(call(coll, x, count, shift, root=root)[rows], expected(coll, x, P, count, root)[rows])
