@@ -1639,13 +1639,16 @@ int launch_copy_units(bine_comm_t c, int mode, dev::CopyArgs a) {
             }
         }
     }
-    // Calls of up to kCopySmallMax elements leave threads idle: with one
-    // element per thread none of them waits for a second load (us, pieces or
-    // realigned vectors / one element: scatter at P = 32 of 192 float32 2.69 /
-    // 2.40, of 1,200 2.30 / 2.05, of 400 off the grid 3.20 / 2.05; alltoall at
-    // P = 4 of 400 off the grid 3.10 / 2.08).  At 303,104 elements, one per
-    // thread that the GPU holds, vectors on the grid lose again.
-    if (!spread && nu >= dev::kCopyBlockMin && units > dev::kCopySmallMax) {
+    // Blocks of at least four threads' elements (us at P = 1000 off the grid,
+    // pieces / one element: 16 bytes 83 / 45, 18 bytes 51 / 51; 16 int32 69 /
+    // 49, 18 int32 45 / 55; 16 int64 107 / 71).  Calls of up to kCopySmallMax
+    // elements leave threads idle: with one element per thread none of them
+    // waits for a second load (us, pieces or realigned vectors / one element:
+    // scatter at P = 32 of 192 float32 2.69 / 2.40, of 1,200 2.30 / 2.05, of 400
+    // off the grid 3.20 / 2.05; alltoall at P = 4 of 400 off the grid 3.10 /
+    // 2.08).  On the grid, 2 to 4 MiB take 0.94 of the pieces' time so, 4 to 8
+    // MiB (from 262,144 vectors) as long as theirs, and more is slower.
+    if (!spread && nu >= (sizeof(U) == 16 ? dev::kCopyVecBlockMin : dev::kCopyBlockMin) && units > dev::kCopySmallMax) {
         // Realigned vectors for 4-byte elements from 1 KiB per block and for
         // narrower ones from 256 bytes; elements otherwise (us, elements /
         // realigned: alltoall at P = 256 with 516-byte blocks 25 / 45, with

@@ -1077,11 +1077,11 @@ __global__ void __launch_bounds__(kThreads, 2048 / kThreads) k_copy_rows(CopyArg
     }
 }
 
-// Blocks of fewer than kCopyBlockMin elements with one destination, and calls
+// Blocks of fewer elements than k_copy_blocks takes, with one destination, and calls
 // of at most kCopySmallMax: up to four elements per thread and round, over
 // the elements of all blocks in order (I: the index type, 32 bits where the
 // element count allows), as many threads as elements where the grid holds them.
-constexpr int kCopySmallMax = 65536;
+constexpr int kCopySmallMax = 262144;
 template <int MODE, typename U, typename I>
 __global__ void __launch_bounds__(kThreads) k_copy_small(CopyArgs a) {
     const I nu = (I)(a.unit / (long long)sizeof(U)), P = (I)a.P;
@@ -1104,14 +1104,15 @@ __global__ void __launch_bounds__(kThreads) k_copy_small(CopyArgs a) {
     }
 }
 
-// Blocks of at least kCopyBlockMin elements with one destination (alltoall,
+// Blocks of at least kCopy[Vec]BlockMin elements with one destination (alltoall,
 // scatter, gather): a group of 2^tp_log2 threads moves a piece of up to E
 // elements per thread, 2^tp_log2 apart, so that a warp's accesses are
 // contiguous runs, E loads are in flight before the stores, and the block
 // numbers are divided out once per thread instead of once per element.
 // Bound by HBM.  Against k_copy (us, B200): alltoall at P = 64 with 64 KiB
 // blocks 89 -> 82, P = 256 with 516-byte blocks 38 -> 25.
-constexpr int kCopyBlockMin = 16;
+constexpr int kCopyBlockMin = 17;     // elements of up to 8 bytes
+constexpr int kCopyVecBlockMin = 16;  // 16-byte vectors
 template <int MODE, typename U>
 __global__ void __launch_bounds__(kThreads) k_copy_blocks(CopyArgs a) {
     constexpr int E = sizeof(U) == 16 ? 4 : 8;

@@ -39,14 +39,23 @@ def test_reduce_scatter_of_whole_vectors(P, vectors, dtype):
 
 
 @pytest.mark.parametrize("dtype,count,shift", [
-    (np.int8, 1021, 1), (np.int8, 1024, 0), (np.int8, 1040, 0), (np.int32, 1024, 1), (np.int32, 1031, 0), (np.int32, 4096, 0),
-    (np.int32, 4100, 0), (np.int64, 1024, 1), (np.int64, 1025, 0)])
+    (np.int8, 4093, 1), (np.int8, 4096, 1), (np.int8, 4097, 0), (np.int32, 4096, 1), (np.int32, 4097, 0), (np.int32, 16384, 0),
+    (np.int32, 16388, 0), (np.int64, 4096, 1), (np.int64, 4097, 0)])
 @pytest.mark.parametrize("coll,P", [("scatter", 64), ("gather", 64), ("alltoall", 8)])
-def test_block_copies_around_65536_elements(coll, P, dtype, count, shift):
-    """64 blocks each: at and below 65,536 elements of the widest type that
+def test_block_copies_around_262144_elements(coll, P, dtype, count, shift):
+    """64 blocks each: at and below 262,144 elements of the widest type that
     fits the call one per thread, above pieces or realigned vectors."""
     root = P - 1
     si, _ = buffer_counts(coll, count, P)
     x = values((P, si), dtype, count)
     rows = [root] if coll == "gather" else slice(None)
     assert np.array_equal(call(coll, x, count, shift, root=root)[rows], expected(coll, x, P, count, root)[rows])
+
+
+@pytest.mark.parametrize("dtype", [np.int8, np.int32, np.int64])
+@pytest.mark.parametrize("count,shift", [(15, 1), (16, 1), (17, 1), (33, 0)])
+def test_many_short_blocks(dtype, count, shift):
+    """Above 262,144 elements, on either side of 16 elements per block."""
+    P = 160
+    x = values((P, P * count), dtype, count)
+    assert np.array_equal(call("alltoall", x, count, shift), expected("alltoall", x, P, count))
