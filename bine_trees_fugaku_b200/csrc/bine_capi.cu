@@ -1614,11 +1614,12 @@ int launch_copy_units(bine_comm_t c, int mode, dev::CopyArgs a) {
     const long long fill = 2LL * dev::kThreads * sms;
     a.by_ranks = dev::FastDiv(a.P, pairs);
     if constexpr (sizeof(U) == 4 || sizeof(U) == 8) {
-        // Broadcasts off the 16-byte grid, from 8 MiB written: below, and
-        // for a few rows, the staging costs more than it gains (us, k_copy
-        // / k_spread: allgather at P = 300, 33 int32 6.3 / 7.5; bcast at
-        // P = 8, 1,000,003 int32 8.5 / 8.9).
-        if (spread && a.P >= 16 && a.P * pairs * a.unit >= (8ll << 20)) {
+        // Broadcasts off the 16-byte grid, from 16 MiB written: below, and
+        // for a few rows, the staging costs more than it gains (us,
+        // k_copy_rows / k_spread: 9 MiB to 16 rows 4.2 / 6.2, to 100 rows 6.2 /
+        // 6.2; 16 MiB to 16 rows 6.2 / 6.2, to 500 rows 8.2 / 7.1; 80 MiB to
+        // 500 rows 26.8 / 16.5; bcast at P = 8, 1,000,003 int32 8.5 / 8.9).
+        if (spread && a.P >= 16 && a.P * pairs * a.unit >= (16ll << 20)) {
             dev::SpreadArgs sa;
             sa.in = mode == dev::kCopyBcast ? a.in + (long long)a.root * a.in_stride : a.in;
             sa.in_stride = a.in_stride;

@@ -59,3 +59,14 @@ def test_many_short_blocks(dtype, count, shift):
     P = 160
     x = values((P, P * count), dtype, count)
     assert np.array_equal(call("alltoall", x, count, shift), expected("alltoall", x, P, count))
+
+
+@pytest.mark.parametrize("coll,P,count,shift", [
+    ("bcast", 16, 262_137, 1), ("bcast", 16, 262_147, 0), ("bcast", 512, 8193, 0), ("allgather", 64, 1023, 1),
+    ("allgather", 64, 1025, 0), ("allgather", 33, 3851, 1), ("allgather", 33, 3853, 0)])
+def test_broadcasts_around_16_mib(coll, P, count, shift):
+    """int32 rows that are stored element by element below, and staged for bulk
+    copies from there on."""
+    si, _ = buffer_counts("allreduce" if coll == "bcast" else coll, count, P)
+    x = values((P, si), np.int32, P + count)
+    assert np.array_equal(call(coll, x, count, shift, root=P - 1), expected(coll, x, P, count, P - 1))
