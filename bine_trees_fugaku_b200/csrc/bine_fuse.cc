@@ -66,10 +66,11 @@ class Exec {
         return id;
     }
     const FNode& node(int32_t id) const { return nodes_[id]; }
-    // Whether every value computed so far is within the fused kernel's bounds.
-    bool within_bounds() {
+    // Whether every value computed so far has at most `max_leaves` leaves (the
+    // same at every call) and fits the fused kernel's stack.
+    bool within_bounds(int max_leaves) {
         for (; checked_ < nodes_.size() && fits_; checked_++)
-            fits_ = nodes_[checked_].leaves <= kFuseMaxLeaves && nodes_[checked_].depth <= kFuseMaxDepth;
+            fits_ = nodes_[checked_].leaves <= max_leaves && nodes_[checked_].depth <= kFuseMaxDepth;
         return fits_;
     }
     void clear_state() { rows_.clear(); }
@@ -279,14 +280,15 @@ struct PassSym {
 };
 
 // Executes levels [a, b); with `end`, stops before the first level after a
-// whose values are too large for the kernel and returns where it stopped.
-PassSym run_pass(const Schedule& sch, int a, int b, int* end = nullptr) {
+// whose values have more than `max_leaves` leaves or are too deep for the
+// kernel, and returns where it stopped.
+PassSym run_pass(const Schedule& sch, int a, int b, int max_leaves = 0, int* end = nullptr) {
     PassSym ps;
     ps.ex.reset(new Exec());
     Exec& ex = *ps.ex;
     for (int l = a; l < b; l++) {
         ex.apply_level(sch.levels[l]);
-        if (end && !ex.within_bounds() && l > a) {
+        if (end && !ex.within_bounds(max_leaves) && l > a) {
             *end = l;
             return run_pass(sch, a, l);
         }
@@ -486,21 +488,29 @@ bool fuse_schedule(const Schedule& sch, int P, int depth, const std::vector<bool
     *out = FusedSchedule();
     const int L = (int)sch.levels.size();
     depth = std::max(1, depth);
-    // A pass ends before the level whose sums outgrow
-    // the kernel's programs, and the next one starts there: early passes as
-    // long as they can be, since the partial sums that a pass writes halve
-    // with each of its levels.  Allreduce B at P = 256 moves 1.13 times the
-    // algorithmic bytes in 3 passes of 5, 6 and 6 levels; passes of 6 levels
-    // halved where they were too large moved 1.34 times in 4 (of 3, 3, 6, 5).  What follows is
-    // cut evenly into as few passes as `depth` allows: at P = 64, 5, 4 and 4
+    // A pass ends before the level whose sums outgrow the kernel's programs,
+    // and the next one starts there: early passes as long as they can be,
+    // since the partial sums that a pass writes halve with each of its levels.
+    // Allreduce B at P = 256 moves 1.13 times the algorithmic bytes in 3
+    // passes of 5, 6 and 6 levels; passes of 6 levels halved where they were
+    // too large moved 1.34 times in 4 (of 3, 3, 6, 5).  What follows is cut
+    // evenly into as few passes as `depth` allows: at P = 64, 5, 4 and 4
     // levels and no results left in slots (4 MiB per rank 126 us, with 5, 6
     // and 2 levels 144).
+    //
+    // From 17 to 32 ranks programs of 8 leaves need no more passes than those
+    // of 16: allreduce B takes 3 either way, and with 16 the second one also
+    // sums, leaves its results in slots, and the third copies them home (us,
+    // 16 leaves / 8: P = 24, 30,000 float32 27.1 / 21.4, 1 MiB of int8 83 / 33;
+    // P = 32, 30,000 float32 24.9 / 20.4).  Up to 16 and from 33 ranks on they
+    // need one or two more (P = 12 to 16: 1.16 times the time).
+    const int max_leaves = P > 16 && P <= 32 ? 8 : kFuseMaxLeaves;
     std::vector<PassSym> ps;
     std::vector<int> pass_levels;
     for (int l = 0, step = depth; l < L;) {
         const int goal = std::min(L, l + step);
         int end = goal;
-        ps.push_back(run_pass(sch, l, goal, &end));
+        ps.push_back(run_pass(sch, l, goal, max_leaves, &end));
         pass_levels.push_back(end - l);
         l = end;
         const int rest = (L - l + depth - 1) / depth;  // passes
