@@ -116,6 +116,7 @@ def lib():
         "bine_comm_set_step_timeout": [vp, ctypes.c_uint],
         "bine_debug_set_barrier_extra": [vp, ctypes.c_uint],
         "bine_debug_set_tree_smem_limit": [vp, sz],
+        "bine_debug_set_link_ring_limit": [vp, i],
         "bine_comm_set_tree_split": [vp, ctypes.c_int],
         "bine_allreduce_host": [vp, vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, vp],
         "bine_allreduce_host_hooked": [vp, vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, vp, WINDOW_HOOK, WINDOW_HOOK,
@@ -295,6 +296,9 @@ class Comm:
 
     def debug_set_tree_smem_limit(self, nbytes):
         check(lib().bine_debug_set_tree_smem_limit(self._h, nbytes))
+
+    def debug_set_link_ring_limit(self, nodes):
+        check(lib().bine_debug_set_link_ring_limit(self._h, nodes))
 
     def synchronize(self):
         check(lib().bine_comm_synchronize(self._h))

@@ -297,6 +297,7 @@ struct bine_comm_s {
     int* status = nullptr;
     unsigned long long step_timeout_ns = 5ull * 1000 * 1000 * 1000;
     unsigned barrier_extra = 0;
+    int link_max_ring = dev::kLinkMaxRing;  // longer rings: k_link_generate
     size_t tree_smem_limit = 227 * 1024;  // static and dynamic, of a tree kernel's block
     // Host-buffer pipeline (bine_allreduce_host), created on first use:
     // copy streams, per-slot events (input copied, reduced, output copied)
@@ -2803,6 +2804,12 @@ int bine_debug_set_barrier_extra(bine_comm_t comm, unsigned extra) {
     return BINE_SUCCESS;
 }
 
+int bine_debug_set_link_ring_limit(bine_comm_t comm, int nodes) {
+    if (!comm || nodes < 0 || nodes > dev::kLinkMaxRing) return fail(BINE_ERR_ARG, "the limit is 0 to 8,192 nodes");
+    comm->link_max_ring = nodes;
+    return BINE_SUCCESS;
+}
+
 int bine_debug_set_tree_smem_limit(bine_comm_t comm, size_t bytes) {
     if (!comm || bytes > 227 * 1024) return fail(BINE_ERR_ARG, "the limit is at most 227 KB");
     comm->tree_smem_limit = bytes;
@@ -3110,7 +3117,7 @@ int bine_link_bytes(bine_comm_t comm, bine_coll_t coll, long count, bine_datatyp
             kind = 2;
     }
     const dev::LinkGen g{t, cf.family, comm->ports, kind, (long long)count, es};
-    if (kind >= 0 && max_ring <= dev::kLinkMaxRing) {
+    if (kind >= 0 && max_ring <= comm->link_max_ring) {
         // One block per ring, writing every link of the ring.
         long long rings = 0;
         for (int d = 0; d < t.ndims; d++) rings += t.size / t.dims[d];

@@ -281,6 +281,11 @@ int bine_debug_set_barrier_extra(bine_comm_t comm, unsigned extra);
  * reduction programs do. */
 int bine_debug_set_tree_smem_limit(bine_comm_t comm, size_t bytes);
 
+/* Debug: the longest torus ring (0 to 8,192 nodes, the default) whose link
+ * loads bine_link_bytes computes ring by ring; generated schedules on tori
+ * with longer ones walk every rank's subtree. */
+int bine_debug_set_link_ring_limit(bine_comm_t comm, int nodes);
+
 /* How the FUSED engine evaluates an exact-order float reduction on a
  * 16-byte-aligned layout, planned on the host only (no device needed;
  * nothing is uploaded or cached):
