@@ -1,11 +1,14 @@
 """Calls on either side of the lines between the kernels for rows and blocks
-off the 16-byte grid, against exact sums and copies."""
+off the 16-byte grid, against exact sums and copies; exact-order sums in place
+and of infinities, NaNs and zeros."""
 import numpy as np
 import pytest
+import torch
 
 import bine_trees_fugaku_b200 as bine
+from oracle import port
 from oracle.common import buffer_counts, expected
-from tests.test_ragged_gpu import call, values
+from tests.test_ragged_gpu import CODE, call, same_bits, values
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +73,53 @@ def test_broadcasts_around_16_mib(coll, P, count, shift):
     si, _ = buffer_counts("allreduce" if coll == "bcast" else coll, count, P)
     x = values((P, si), np.int32, P + count)
     assert np.array_equal(call(coll, x, count, shift, root=P - 1), expected(coll, x, P, count, P - 1))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("P,count,lanes", [(4, 1, 0), (24, 2051, 0), (96, 4097, 2), (64, 1027, 8), (200, 601, 0)])
+def test_exact_order_allreduce_in_place_off_the_grid(P, count, lanes, dtype):
+    """Input and output are one array of packed rows of odd length."""
+    if count < P:  # the bandwidth-optimal schedule needs a block per rank
+        count += P
+    x = values((P, count), dtype, P + count)
+    want, _ = port.run("allreduce", x, count, variant="B")
+    buf = torch.from_numpy(x).cuda()
+    comm = bine.Comm(P)
+    comm.set_algo("allreduce", "B")
+    comm.set_tree_split(lanes)
+    comm.set_stream(torch.cuda.current_stream())
+    comm.allreduce(buf, buf, count, CODE[np.dtype(dtype)])
+    comm.synchronize()
+    assert same_bits(buf.cpu().numpy(), want)
+    comm.close()
+
+
+@pytest.mark.parametrize("engine", ["fused", "pipelined"])
+@pytest.mark.parametrize("P,count,lanes", [(16, 131, 0), (24, 67, 0), (96, 389, 4), (64, 256, 0)])
+def test_infinities_nans_and_signed_zeros(P, count, lanes, engine):
+    """Columns of infinities of one and of both signs, a NaN, and zeros of
+    either sign only: the reference's order gives the same class of result,
+    and the same bits where it is a number."""
+    x = values((P, count), np.float32, P)
+    x[P // 2, 0::7] = np.inf
+    x[P - 1, 1::7] = -np.inf
+    x[0, 2::7], x[P // 3, 2::7] = np.inf, -np.inf
+    x[1, 3::7] = np.nan
+    x[:, 4::7] = -0.0
+    x[:, 5::7] = 0.0
+    x[::2, 5::7] = -0.0
+    with np.errstate(invalid="ignore"):
+        want, _ = port.run("allreduce", x, count, variant="B")
+    comm = bine.Comm(P)
+    comm.set_algo("allreduce", "B")
+    comm.set_engine(engine)
+    comm.set_tree_split(lanes)
+    comm.set_stream(torch.cuda.current_stream())
+    send = torch.from_numpy(x).cuda()
+    recv = torch.zeros_like(send)
+    comm.allreduce(send, recv, count, bine.FLOAT)
+    comm.synchronize()
+    got = recv.cpu().numpy()
+    comm.close()
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.isnan(want[:, 2::7]).all()
+    assert np.array_equal(got.view(np.uint32)[~np.isnan(want)], want.view(np.uint32)[~np.isnan(want)])
