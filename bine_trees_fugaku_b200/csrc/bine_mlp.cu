@@ -545,7 +545,7 @@ struct bine_mlp_s {
     bf16* act[3] = {nullptr};    // hidden activations (bf16)
     bf16* dpre[2] = {nullptr};   // bf16 gradients of two consecutive layers
     int* counts = nullptr;       // valid targets per prepare block
-    float* losses = nullptr;     // loss per output tile, then the loss
+    float* losses = nullptr;     // loss per output tile, then the loss, then `side`
     float* loss = nullptr;
     float* side = nullptr;       // output, or targets and mask, where the caller's are not this device's
     float* staged = nullptr;     // pinned host copy of the gradients and the loss
@@ -562,7 +562,6 @@ struct bine_mlp_s {
         for (bf16* p : dpre) cudaFree(p);
         cudaFree(counts);
         cudaFree(losses);
-        cudaFree(side);
         cudaFreeHost(staged);
         if (inputs_read) cudaEventDestroy(inputs_read);
     }
@@ -730,9 +729,10 @@ int bine_mlp_create(int in_dim, int hidden, int out_dim, int max_batch, unsigned
         MLP_TRY(cudaMalloc(&m->dpre[l], (size_t)max_batch * std::max(hidden, out_dim) * sizeof(bf16)));
     MLP_TRY(cudaMalloc(&m->counts, kPrepBlocks * sizeof(int)));
     const size_t nlosses = (size_t)tiles(max_batch) * tiles(out_dim);
-    MLP_TRY(cudaMalloc(&m->losses, (nlosses + 1) * sizeof(float)));
+    const size_t aside = (nlosses + 1 + 3) / 4 * 4;  // a 16-byte boundary
+    MLP_TRY(cudaMalloc(&m->losses, (aside + 2 * (size_t)max_batch * out_dim) * sizeof(float)));
     m->loss = m->losses + nlosses;
-    MLP_TRY(cudaMalloc(&m->side, 2 * (size_t)max_batch * out_dim * sizeof(float)));
+    m->side = m->losses + aside;
     MLP_TRY(cudaMallocHost(&m->staged, (off + 1) * sizeof(float)));
     MLP_TRY(cudaEventCreateWithFlags(&m->inputs_read, cudaEventDisableTiming));
     MLP_TRY(cudaDeviceSynchronize());
