@@ -2375,8 +2375,8 @@ struct bine_batch_s {
 namespace {
 
 // Grid: up to 16 times the resident blocks, back-filled by the hardware as
-// blocks finish (512 mixed calls of up to 64 KiB, 1.97 GB: 416 us with the
-// resident blocks alone, 363 with 16 times as many).
+// blocks finish (512 mixed calls of up to 64 KiB, 1.97 GB: 386 us with the
+// resident blocks alone, 340 with four times as many, 333 with 16 times).
 const bine_batch_tuning_t kDefaultTuning = {{8, 32, 128, 1 << 30}, {256, 128, 64, 32}, 16, 1};
 
 int batch_layout(const bine_batch_item_t* items, int n, const bine_batch_tuning_t& tu,

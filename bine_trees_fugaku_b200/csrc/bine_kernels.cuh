@@ -61,8 +61,9 @@ __device__ __forceinline__ void st_stream(void* p, uint4 v) {
 // Strided lane vectors, for rows that do not share a 16-byte grid (packed
 // rows of odd length, blocks of odd length): the 16 / sizeof(T) elements of
 // a lane lie `STEP` elements apart and consecutive lanes hold consecutive
-// elements, so every access of a warp is a run of 32 elements wherever the
-// row starts, and the vector arithmetic stays that of the 16-byte form.
+// elements, so every access of a warp is runs of min(32, STEP) elements
+// wherever the row starts, and the vector arithmetic stays that of the 16-byte
+// form.
 // `n` elements of the vector exist (the first ones); the others read as 0.
 template <typename T>
 __device__ __forceinline__ T ld_stream_elem(const void* p) {
@@ -188,13 +189,14 @@ enum SumMode { kSumAllreduce = 0, kSumReduceScatter = 1, kSumReduce = 2 };
 // reduce_scatter: `blk` elements per destination rank, and `in` is element
 // `e0` of the row.  VEC: lane vectors of 16 contiguous, aligned bytes (n is
 // whole vectors, blk counts vectors, e0 is 0; with blk in elements int8 at P =
-// 768 and 16 elements took 7.6 us, 6.5 so).  Otherwise strided ones (ld_strided, COLS elements
-// apart), for rows off the 16-byte grid and for the last partial vector:
-// the loop over the rows is the same, with four loads of 4 bytes in the
-// place of one of 16.  They replaced one thread per element with its P rows
-// in a chain (int32 allreduce, us per call): P = 96 at 262,147 elements per
-// rank 47.7 -> 39.3 (37.3 at 262,144, on the grid), P = 256 at 1,048,577
-// 509 -> 381, P = 300 at 777 int64 28.3 -> 8.1, P = 500 at 1 15.0 -> 7.3.
+// 768 and 16 elements took 7.6 us, 6.5 so).  Otherwise strided ones
+// (ld_strided, COLS elements apart), for rows off the 16-byte grid and for the
+// last partial vector of 16 ranks and more: the loop over the rows is the
+// same, with four loads of 4 bytes in the place of one of 16, bound by their
+// issue.  They replaced one thread per element with its P rows in a chain
+// (int32 allreduce, us per call): P = 96 at 262,147 elements per rank 47.7 ->
+// 39.3 (37.3 at 262,144, on the grid), P = 256 at 1,048,577 509 -> 381, P =
+// 300 at 777 int64 28.3 -> 8.1, P = 500 at 1 15.0 -> 7.3.
 constexpr int kSumCols = 8;  // the narrowest tile (32 row groups)
 
 template <typename T, int MODE, int COLS, bool VEC>
@@ -886,9 +888,12 @@ __global__ void __launch_bounds__(kThreads) k_tree_staged(const char* __restrict
 // first, so every load and store of a warp is one run of 32 elements.  K = 1
 // evaluates whole programs (no split plan).
 //
-// Bound by HBM like the aligned form (the arithmetic per row is the same,
-// with four 4-byte loads in the place of one of 16).  It replaced a kernel
-// of one element per thread and one load in flight on 1,024-element tiles
+// The arithmetic per row is that of the aligned form, with four 4-byte loads
+// in the place of one of 16: bound by the latency and the issue of those
+// loads at four blocks of 64 registers per SM (42 % of the warps; float32 at
+// P = 96, 262,147 elements: DRAM and L1 at 42 and 43 % of their peaks, 70 % of
+// the copy rate; most stalled on loads in flight).  It replaced a kernel of
+// one element per thread and one load in flight on 1,024-element tiles
 // (288 blocks): float32 allreduce at P = 96, 262,147 elements per rank,
 // 232 -> 44.3 us per call (867 -> 4,550 GB/s); P = 256 at 1,048,579
 // elements runs at 5,180 GB/s, reduce_scatter at P = 64 and 32,769 at 5,530.
@@ -1005,7 +1010,7 @@ struct CopyArgs {
     int P;
     int root;
     long long unit;    // bytes per block
-    int dgroups;       // k_copy, allgather / bcast: destination groups per source element (>= 1)
+    int dgroups;       // k_copy_rows (allgather, bcast): destination groups per source element (>= 1)
     // k_copy_blocks, k_copy_shift: a pair is cut into `chunks` pieces.
     long long groups;  // pairs * chunks
     long long chunks;
@@ -1110,8 +1115,9 @@ __global__ void __launch_bounds__(kThreads) k_copy_small(CopyArgs a) {
 // elements per thread, 2^tp_log2 apart, so that a warp's accesses are
 // contiguous runs, E loads are in flight before the stores, and the block
 // numbers are divided out once per thread instead of once per element.
-// Bound by HBM.  Against k_copy (us, B200): alltoall at P = 64 with 64 KiB
-// blocks 89 -> 82, P = 256 with 516-byte blocks 38 -> 25.
+// Bound by HBM.  Against one element per thread and grid step (us, B200):
+// alltoall at P = 64 with 64 KiB blocks 89 -> 82, P = 256 with 516-byte blocks
+// 38 -> 25.
 constexpr int kCopyBlockMin = 17;     // elements of up to 8 bytes
 constexpr int kCopyVecBlockMin = 16;  // 16-byte vectors
 template <int MODE, typename U>
@@ -1147,10 +1153,11 @@ __global__ void __launch_bounds__(kThreads) k_copy_blocks(CopyArgs a) {
 // bytes before and after it are element stores.  Rows are split into groups
 // to give the GPU about kSpreadItems blocks per SM.
 //
-// Bound by HBM writes: element stores off the grid leave two partial
-// sectors per 128 bytes.  Measured on B200 (us): bcast at P = 96,
+// Bound by HBM writes (bcast at P = 96, 1,000,001 int32: 87 % of the copy
+// rate): element stores off the grid leave two partial sectors per 128 bytes.
+// Measured on B200 (us): bcast at P = 96,
 // 1,000,001 int32 116 -> 73, allgather at P = 41, 20,001 floats 40.1 ->
-// 28.5.  Rows on the grid need no staging and stay with k_copy (allgather
+// 28.5.  Rows on the grid need no staging and stay with k_copy_rows (allgather
 // at P = 96, 32 KiB: 52.4 there, 58 here).
 constexpr int kSpreadThreads = 128;
 constexpr int kSpreadTile = 4096;  // bytes of the sequence per block
@@ -1227,8 +1234,10 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread(const SpreadArgs a) {
 // are read, so up to 31 bytes at a block's start and 47 at its end are
 // copied as elements of type U.
 //
-// Bound by HBM: whole-sector stores, where element stores off the grid leave
-// two partial sectors per 128 bytes.  Measured on B200 (us, one element per
+// Stores are whole sectors, where element stores off the grid leave two
+// partial sectors per 128 bytes.  Bound by load latency: 78 registers for
+// 4-byte elements leave three blocks per SM (30 % of the warps; DRAM at 57 % of
+// its peak, 78 % of the copy rate).  Measured on B200 (us, one element per
 // thread -> this kernel): alltoall at P = 64 with blocks of 10,001 int32 158
 // -> 64, of 10,001 bytes 153 -> 18.8; P = 128 with 2,052-byte blocks 37.4 ->
 // 16.7.
@@ -2355,10 +2364,10 @@ __global__ void k_link_scan(Torus t, unsigned long long* links) {
 // tile a few tiles of 2 MB ended a small batch (64 calls, 55 MB: 49 us).
 // Integer sums wrap, float32 sums accumulate in FP64 (the FAST order).
 //
-// Bound by HBM.  B200, us per launch with the default tuning, start -> now
-// (of which the larger grid alone took the first to 363): 512 mixed calls
-// of up to 64 KiB (1.97 GB) 416 -> 345, 1,000 of up to 2 KiB (0.97 GB) 209 ->
-// 170, 64 of up to 4 KiB (55 MB) 49 -> 14.6.
+// Bound by HBM.  B200, us per launch with the default tuning, against tiles of
+// all rows, a search of all calls and a grid of the resident blocks: 512 mixed
+// calls of up to 64 KiB (1.97 GB) 386 -> 333, 400 of up to 500 bytes on up to
+// 512 ranks 98.9 -> 68.0, 60 of those 39.0 -> 16.5.
 namespace bine {
 namespace dev {
 

@@ -154,9 +154,11 @@ int bine_comm_set_segment(bine_comm_t comm, long long segment_bytes);
  * in its slot, what the reference's buffers hold after that step.  No
  * counterpart in the reference.  0 chooses the levels per pass for each
  * collective (allreduce, reduce_scatter and reduce 6; allgather, bcast,
- * scatter and gather 12; alltoall 13) and runs schedules of more than 2^20
- * moves level by level: planning a fused schedule costs about 4 us per move
- * on the host, once per call shape. */
+ * scatter and gather 12; alltoall 13; on up to 8 ranks all levels at once,
+ * where that is more) and runs schedules of more than 2^20 moves level by
+ * level.  A pass ends earlier, before the level whose sums would have more
+ * terms than the kernel's programs hold.  Planning a fused schedule costs
+ * about 4 us per move on the host, once per call shape. */
 int bine_comm_set_fusion(bine_comm_t comm, int levels);
 int bine_comm_set_float_order(bine_comm_t comm, int order);
 
@@ -320,8 +322,8 @@ int bine_comm_set_tree_split(bine_comm_t comm, int lanes);
 /* ------------------------------------------------------------- batching
  * Many independent allreduce / reduce_scatter / allgather calls of
  * different rank counts, sizes and element types (BINE_INT32 or
- * BINE_FLOAT) executed by ONE persistent kernel launch, which can be
- * captured in a CUDA graph.  Each item is a complete collective over its
+ * BINE_FLOAT) executed by ONE kernel launch (by default of up to 16 times the
+ * blocks that fit on the GPU at once), which can be captured in a CUDA graph.  Each item is a complete collective over its
  * own `nranks` virtual ranks, with the argument meaning of its entry point
  * (count = allreduce count, reduce_scatter recvcount, allgather
  * sendcount).  Rows must be 16-byte aligned and hold whole 16-byte vectors
@@ -359,7 +361,7 @@ typedef struct bine_batch_s *bine_batch_t;
  * (tuning NULL: defaults). */
 int bine_batch_create(const bine_batch_item_t *items, int nitems, const bine_batch_tuning_t *tuning,
                       bine_batch_t *batch);
-/* One persistent launch of the whole batch on `stream` (capturable). */
+/* One launch of the whole batch on `stream` (capturable). */
 int bine_batch_launch(bine_batch_t batch, void *stream);
 int bine_batch_destroy(bine_batch_t batch);
 /* Times candidate tunings of this batch on `stream` (reps launches each,
