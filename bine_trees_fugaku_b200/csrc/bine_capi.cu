@@ -1303,8 +1303,16 @@ int launch_sum(bine_comm_t c, int mode, const char* in, long long ist, char* out
     // per element, int32 allreduce: P = 4, 1 element 1.95 / 1.73; P = 8, 20,001
     // 2.88 / 2.59; P = 12, 300,001 5.95 / 5.66; float32 in the FAST order, P = 9,
     // 672,944 12.4 / 8.3).  At P = 16 the two are equal for rows in L2 and the
-    // vectors 10 % faster for rows outside it.
-    if (sizeof(T) == 1 || c->P < 16) {
+    // vectors 10 % faster for rows outside it.  With more than 65,536 elements
+    // the threads alone fill the GPU, and four loads for each vector and row
+    // cost more than they save up to about 24 ranks, in allreduce (whose
+    // stores are as many) 40: strided over per element, rows in L2 / outside it,
+    // geometric means over 65,537 to 1,048,577 elements of 4 and 8 bytes:
+    // allreduce P = 24 1.32 / 1.11, P = 40 1.19 / 1.02, P = 64 1.07 / 0.94;
+    // reduce P = 24 1.48 / 1.06, P = 48 1.25 / 0.91; reduce_scatter P = 24 1.40 /
+    // 1.07, P = 32 1.16 / 0.91.
+    const bool few_rows = c->P < 16 || (rest > dev::kSumManyElems && c->P <= (mode == dev::kSumAllreduce ? 40 : 24));
+    if (sizeof(T) == 1 || few_rows) {
         const unsigned g = grid_for(c, rest);
         if (mode == dev::kSumAllreduce)
             dev::k_sum_scalar<T, dev::kSumAllreduce><<<g, dev::kThreads, 0, c->stream>>>(in, ist, out, ost, c->P, done, rest, blk, root);

@@ -191,7 +191,7 @@ enum SumMode { kSumAllreduce = 0, kSumReduceScatter = 1, kSumReduce = 2 };
 // whole vectors, blk counts vectors, e0 is 0; with blk in elements int8 at P =
 // 768 and 16 elements took 7.6 us, 6.5 so).  Otherwise strided ones
 // (ld_strided, COLS elements apart), for rows off the 16-byte grid and for the
-// last partial vector of 16 ranks and more: the loop over the rows is the
+// last partial vector, except for few ranks: the loop over the rows is the
 // same, with four loads of 4 bytes in the place of one of 16, bound by their
 // issue.  They replaced one thread per element with its P rows in a chain
 // (int32 allreduce, us per call): P = 96 at 262,147 elements per rank 47.7 ->
@@ -277,11 +277,12 @@ __global__ void __launch_bounds__(kThreads) k_sum_vec(const char* __restrict__ i
     }
 }
 
-// Sums off the 16-byte grid of 1-byte elements and of fewer than 16 ranks,
-// elements [e0, e0 + n) of every row, one per thread: a strided lane vector of
-// bytes would take 16 loads of one byte each (int8 allreduce at P = 96,
-// 262,147 elements per rank: 20.7 us here, 33.3 us strided), and with few rows
-// one thread's loads are few.  reduce_scatter: `blk` elements per rank.
+// Sums off the 16-byte grid of 1-byte elements and of few ranks, elements [e0,
+// e0 + n) of every row, one per thread: a strided lane vector of bytes would
+// take 16 loads of one byte each (int8 allreduce at P = 96, 262,147 elements
+// per rank: 20.7 us here, 33.3 us strided), and with few rows one thread's
+// loads are few.  reduce_scatter: `blk` elements per rank.
+constexpr int kSumManyElems = 65536;  // from here on few ranks are up to 24 or 40 (launch_sum)
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kThreads) k_sum_scalar(const char* __restrict__ in, long long in_stride,
                                                          char* __restrict__ out, long long out_stride, int P,

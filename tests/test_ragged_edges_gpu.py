@@ -123,3 +123,17 @@ def test_infinities_nans_and_signed_zeros(P, count, lanes, engine):
     comm.close()
     assert np.array_equal(np.isnan(got), np.isnan(want)) and np.isnan(want[:, 2::7]).all()
     assert np.array_equal(got.view(np.uint32)[~np.isnan(want)], want.view(np.uint32)[~np.isnan(want)])
+
+
+@pytest.mark.parametrize("coll,P", [("allreduce", 40), ("allreduce", 41), ("reduce", 24), ("reduce", 25),
+                                    ("reduce_scatter", 24), ("reduce_scatter", 25)])
+@pytest.mark.parametrize("extra", [-2, 3])
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+def test_sums_of_few_ranks_around_65536_elements(coll, P, extra, dtype):
+    """One element per thread above 65,536 elements up to 40 (24) ranks,
+    strided vectors below and beyond."""
+    count = 65536 + extra if coll != "reduce_scatter" else 65536 // P + extra
+    si, _ = buffer_counts(coll, count, P)
+    x = values((P, si), dtype, P + extra)
+    rows = [0] if coll == "reduce" else slice(None)
+    assert np.array_equal(call(coll, x, count, 1)[rows], expected(coll, x, P, count, 0)[rows])
