@@ -2367,8 +2367,8 @@ __global__ void k_link_scan(Torus t, unsigned long long* links) {
 //
 // Bound by HBM.  B200, us per launch with the default tuning, against tiles of
 // all rows, a search of all calls and a grid of the resident blocks: 512 mixed
-// calls of up to 64 KiB (1.97 GB) 386 -> 333, 400 of up to 500 bytes on up to
-// 512 ranks 98.9 -> 68.0, 60 of those 39.0 -> 16.5.
+// calls of up to 64 KiB (1.97 GB) 386 -> 332, 400 of up to 500 bytes on up to
+// 512 ranks 98.8 -> 61.6, 60 of those 39.0 -> 16.4.
 namespace bine {
 namespace dev {
 
@@ -2433,8 +2433,12 @@ __device__ __forceinline__ void batch_reduce_tile(const BatchItem& it, long long
     }
 }
 
+// Four blocks per SM: 64 registers keep a reduction tile's eight loads in
+// flight.  With the 46 to 48 that the compiler takes unasked, float tiles of
+// many rows wait for them in turn (us, 48 registers / 64: one call of 888 floats
+// on 456 ranks 14.4 / 10.9, of 40 floats on 521 ranks outside L2 26.6 / 14.5).
 template <bool TABLE>
-__global__ void __launch_bounds__(kThreads) k_batch(const BatchItem* __restrict__ items, int nitems,
+__global__ void __launch_bounds__(kThreads, 4) k_batch(const BatchItem* __restrict__ items, int nitems,
                                                     const int* __restrict__ hint, long long total_tiles) {
     __shared__ Lanes<float, double> part[kThreads];
     __shared__ uint4 res[kThreads];

@@ -28,3 +28,24 @@ def test_batches_around_the_table_size(calls, vectors):
     for k in range(calls):
         assert np.array_equal(outs[k].cpu().numpy().reshape(wants[k].shape), wants[k]), k
     b.close()
+
+
+@pytest.mark.parametrize("P,count", [(456, 888), (521, 40), (97, 4), (1024, 8)])
+@pytest.mark.parametrize("coll", ["allreduce", "reduce_scatter"])
+def test_float_tiles_of_many_rows(coll, P, count):
+    """FP64 accumulation and one rounding: within half an ulp of the FP64 sum
+    and that sum's own P 2^-52 sum|x|."""
+    from oracle.common import buffer_counts
+
+    if coll == "reduce_scatter":
+        count = 4
+    si, so = buffer_counts(coll, count, P)
+    x = np.random.default_rng(P).standard_normal((P, si)).astype(np.float32)
+    y = torch.zeros((P, so), device="cuda")
+    b = bine.Batch([(coll, torch.from_numpy(x).cuda(), y, count, bine.FLOAT, P)])
+    b.launch()
+    torch.cuda.synchronize()
+    want = expected(coll, x.astype(np.float64), P, count)
+    absum = expected(coll, np.abs(x).astype(np.float64), P, count)
+    assert np.all(np.abs(y.cpu().numpy().reshape(want.shape) - want) <= np.abs(want) * 2.0 ** -24 + P * 2.0 ** -52 * absum)
+    b.close()
